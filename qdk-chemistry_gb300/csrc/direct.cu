@@ -25,10 +25,12 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <unordered_map>
 #include <vector>
 
 #include "common.cuh"
+#include "contract.cuh"
 #include "internal.h"
 #include "tcgen05.cuh"
 
@@ -94,7 +96,9 @@ struct SpinTables {
   int ns = 0, nd = 0;
   DeviceBuffer sJ, svo, dJ, dvo, packed, str;
   DeviceBuffer sA64, sA32, dval64, dval32, W64, W32;
-  std::vector<uint32_t> h_packed;  // host copy of `packed` while the contraction tables are built
+  // host copies of `packed` and `dJ` while the contraction tables are built
+  std::vector<uint32_t> h_packed;
+  std::vector<int32_t> h_dJ;
 };
 
 struct DirectSigma {
@@ -142,6 +146,15 @@ struct DirectSigma {
   DeviceBuffer HaaS, HbbS, XA, XB;
   int nkb1 = 0, nkb2 = 0;
   int64_t szA1 = 0, szB1 = 0, szA2 = 0, szB2 = 0;  // floats per split part
+  // the contraction from 16-bit parts (contract.cuh): structure for both
+  // precisions (ct), the pair rows, the walk lists per chunk of beta strings;
+  // values for integrals with V(..|rs) = V(..|sr) (use32 / use64)
+  bool ct = false, use32 = false, use64 = false;
+  int ct_mr = 0, ct_R = 0, ct_kpad = 0, ct_nbp = 0, ct_seg = 0;
+  int dn_flush = 0;
+  unsigned* ct_fault = nullptr;  // g_tc_fault's device address
+  DeviceBuffer ct_rs, ct_walk, ct_segs, ct_V32, ct_V64, ct_C, ct_rexp, ct_cexp, ct_flag;
+  DeviceBuffer dn_Ha, dn_Hb, dn_ea, dn_eb, dn_CA, dn_CB;
   // batched CASCI over instances of this space (direct_batch_*): per-instance
   // FP32 value tables and their dense same-spin matrices; bform -1 until the
   // first call fixes the contraction form (0 FMA pipe, 1 tensor cores)
@@ -159,7 +172,9 @@ void free_direct(Context* c) {
   for (DeviceBuffer* b : {&d->V32, &d->tmp64, &d->tmp32, &d->ct64, &d->ct32, &d->V2mm, &d->rs_of, &d->lists, &d->seg,
                           &d->Haa, &d->HbbT, &d->bsAa, &d->bWa, &d->bdva, &d->bsAb, &d->bWb, &d->bdvb, &d->bV2,
                           &d->bHaa, &d->bHbbT, &d->HaaS, &d->HbbS, &d->XA, &d->XB, &d->bHaaS, &d->bHbbS,
-                          &d->bXA, &d->bXB})
+                          &d->bXA, &d->bXB, &d->ct_rs, &d->ct_walk, &d->ct_segs, &d->ct_V32, &d->ct_V64, &d->ct_C,
+                          &d->ct_rexp, &d->ct_cexp, &d->ct_flag, &d->dn_Ha, &d->dn_Hb, &d->dn_ea, &d->dn_eb,
+                          &d->dn_CA, &d->dn_CB})
     dev_free(c, *b);
   delete d;
   c->direct = nullptr;
@@ -228,6 +243,7 @@ static void build_spin_tables(Context* c, const std::vector<uint64_t>& strs, Spi
   up(t.str, strs.data(), strs.size() * 8);
   QDKGB_CUDA(cudaStreamSynchronize(c->stream));
   t.h_packed = std::move(packed);
+  t.h_dJ = std::move(dJ);
 }
 
 // Values of one spin's tables from the integrals, in the order of the
@@ -1196,9 +1212,21 @@ static void tune_recall(Context* c, DirectSigma* d) {
     }
 }
 
+static void ct_sigma64(Context* c, const double* x, double* y);
+template <typename T>
+static ct::Args<T> ct_args(Context* c, DirectSigma* d, const T* x, T* y);
+template <typename T>
+static void ct_launch(Context* c, const ct::Args<T>& g, int B);
+
 template <typename T>
 static void direct_sigma_t(Context* c, const T* x, T* y) {
   DirectSigma* d = c->direct;
+  if constexpr (sizeof(T) == 8) {
+    if (d->use64) {
+      ct_sigma64(c, x, y);
+      return;
+    }
+  }
   const SpinTables& A = d->a;
   const SpinTables& B = d->same ? d->a : d->b;
   const int64_t na = A.nstr, nb = B.nstr, N = na * nb;
@@ -1270,8 +1298,17 @@ static void direct_sigma_t(Context* c, const T* x, T* y) {
             (const float*)d->V2mm.ptr, d->n, (const double*)c->H.diag.ptr, (const float*)x, (float*)y);
       };
       // the contraction into yo (which reads yo as its start value): the
-      // FMA-pipe kernel (0) or the tensor-core one (1)
+      // FMA-pipe kernel (0), the TF32 tensor-core one (1) or the one from
+      // bfloat16 parts (2)
       auto contract = [&](float* yo, int form) {
+        if (form == 2) {
+          ct::Args<float> g = ct_args<float>(c, d, (const float*)x, yo);
+          ct::k_ct_split32<<<(unsigned)na, 256, 0, c->stream>>>((int)nb, d->ct_nbp, g.part, (const float*)x,
+                                                                (uint16_t*)d->ct_C.ptr, 0, 0, nullptr);
+          QDKGB_CHECK_LAUNCH();
+          ct_launch(c, g, 1);
+          return;
+        }
         if (form == 1) {
           auto gt = [&](auto kern) {
             kern<<<(unsigned)na, kOtThreads + 32, d->otc_smem, c->stream>>>(
@@ -1318,7 +1355,7 @@ static void direct_sigma_t(Context* c, const T* x, T* y) {
         }
         QDKGB_CHECK_LAUNCH();
       };
-      if (d->otc && d->otc_state < 0) {
+      if (!d->use32 && d->otc && d->otc_state < 0) {
         // first FP32 sigma of this space: time both contractions on a copy
         // of the same-spin result and keep the faster
         float* sc = (float*)dev_alloc(c, d->tmp32, N * sizeof(float));
@@ -1344,7 +1381,7 @@ static void direct_sigma_t(Context* c, const T* x, T* y) {
         d->otc_state = d->otc_ms[1] < d->otc_ms[0] ? 1 : 0;
         tune_record(c, d);
       }
-      contract((float*)y, d->otc && d->otc_state == 1 ? 1 : 0);
+      contract((float*)y, d->use32 ? 2 : d->otc && d->otc_state == 1 ? 1 : 0);
       QDKGB_CHECK_LAUNCH();
       return;
     }
@@ -1371,10 +1408,188 @@ __global__ void k_diag_product(Integrals I, int64_t na, int64_t nb, const uint64
   }
 }
 
+// Values of the contraction from 16-bit parts: its V tables, the FP64 dense
+// matrices' digits; d->use32 / d->use64 where the integrals allow the form.
+static void ct_values(Context* c, DirectSigma* d) {
+  d->use32 = d->use64 = false;
+  if (!d->ct || !d->tc || d->mm_env == '0') return;
+  const int n = d->n;
+  const int64_t n4 = (int64_t)n * n * n * n, n2 = (int64_t)n * n;
+  const SpinTables& A = d->a;
+  const SpinTables& B = d->same ? d->a : d->b;
+  const int64_t na = A.nstr, nb = B.nstr;
+  const int nkb1 = (int)((na + ct::kDnK - 1) / ct::kDnK), nkb2 = (int)((nb + ct::kDnK - 1) / ct::kDnK);
+  const int64_t ta = (na + ct::kDnM - 1) / ct::kDnM, tb = (nb + ct::kDnN - 1) / ct::kDnN;
+  if (c->dev_limit > 0) {
+    // a capped context keeps the memory it had for a Davidson workspace of any
+    // size: the 16-bit operands only beside that
+    const double need = 14.0 * na * d->ct_nbp + (double)(ta * ct::kDnA) * (nkb1 + nkb2) +
+                        (double)(tb * ct::kDnB) * (nkb1 + nkb2) + 64.0 * (na + nb);
+    if (need + 8.0 * na * nb * 530 > (double)(c->dev_limit - c->dev_bytes)) return;
+  }
+  int* flag = dev_array<int>(c, d->ct_flag, 2);  // [0] asymmetric integrals, [1] non-finite vector
+  QDKGB_CUDA(cudaMemsetAsync(flag, 0, 8, c->stream));
+  const unsigned blk = (unsigned)std::min<int64_t>((n4 + 255) / 256, (int64_t)c->sm_count * 8);
+  ct::k_ct_symmetry<<<blk, 256, 0, c->stream>>>((const double*)c->V.ptr, n, n4, flag);
+  QDKGB_CHECK_LAUNCH();
+  int h = 0;
+  QDKGB_CUDA(cudaMemcpyAsync(&h, flag, 4, cudaMemcpyDeviceToHost, c->stream));
+  float* v32 = dev_array<float>(c, d->ct_V32, (size_t)(n2 * d->ct_R));
+  double* v64 = dev_array<double>(c, d->ct_V64, (size_t)(n2 * d->ct_R));
+  const unsigned b2 = (unsigned)std::min<int64_t>((n2 * d->ct_R + 255) / 256, (int64_t)c->sm_count * 8);
+  ct::k_ct_v2<float><<<b2, 256, 0, c->stream>>>((const double*)c->V.ptr, (const int32_t*)d->ct_rs.ptr, n, d->ct_mr,
+                                                d->ct_R, v32);
+  QDKGB_CHECK_LAUNCH();
+  ct::k_ct_v2<double><<<b2, 256, 0, c->stream>>>((const double*)c->V.ptr, (const int32_t*)d->ct_rs.ptr, n, d->ct_mr,
+                                                 d->ct_R, v64);
+  QDKGB_CHECK_LAUNCH();
+  dev_array<uint16_t>(c, d->ct_C, (size_t)(7 * na * d->ct_nbp));
+  void* fault = nullptr;
+  QDKGB_CUDA(cudaGetSymbolAddress(&fault, g_tc_fault));
+  d->ct_fault = (unsigned*)fault;
+  QDKGB_CUDA(cudaStreamSynchronize(c->stream));
+  d->use32 = !(h & 2);
+  if ((h & 1) || d->dn_flush < 1) return;
+  uint16_t* Ha = dev_array<uint16_t>(c, d->dn_Ha, (size_t)(ta * nkb1 * ct::kDnA / 2));
+  uint16_t* Hb = dev_array<uint16_t>(c, d->dn_Hb, (size_t)(tb * nkb2 * ct::kDnB / 2));
+  dev_array<uint16_t>(c, d->dn_CA, (size_t)(ta * nkb2 * ct::kDnA / 2));
+  dev_array<uint16_t>(c, d->dn_CB, (size_t)(tb * nkb1 * ct::kDnB / 2));
+  int* ea = dev_array<int>(c, d->dn_ea, (size_t)na);
+  int* eb = dev_array<int>(c, d->dn_eb, (size_t)nb);
+  dev_array<int>(c, d->ct_rexp, (size_t)na);
+  dev_array<int>(c, d->ct_cexp, (size_t)nb);
+  QDKGB_CUDA(cudaMemsetAsync(Ha, 0, (size_t)(ta * nkb1 * ct::kDnA), c->stream));
+  QDKGB_CUDA(cudaMemsetAsync(Hb, 0, (size_t)(tb * nkb2 * ct::kDnB), c->stream));
+  ct::k_dn_matrix<<<(unsigned)na, 128, 0, c->stream>>>(A.nd, 0, (const int32_t*)A.dJ.ptr, (const double*)A.dval64.ptr,
+                                                       nullptr, nullptr, nullptr, ct::kDnM, nkb1, Ha, ea);
+  QDKGB_CHECK_LAUNCH();
+  ct::k_dn_matrix<<<(unsigned)nb, 128, 0, c->stream>>>(
+      B.nd, B.ns, (const int32_t*)B.dJ.ptr, (const double*)B.dval64.ptr, (const int32_t*)B.sJ.ptr,
+      (const int32_t*)B.svo.ptr, (const double*)B.sA64.ptr, ct::kDnN, nkb2, Hb, eb);
+  QDKGB_CHECK_LAUNCH();
+  set_max_dynamic_smem((const void*)ct::k_dense64, ct::kDnStages * (ct::kDnA + ct::kDnB));
+  d->use64 = true;
+}
+
+template <typename T>
+static ct::Args<T> ct_args(Context* c, DirectSigma* d, const T* x, T* y) {
+  const SpinTables& A = d->a;
+  const SpinTables& B = d->same ? d->a : d->b;
+  const bool f64 = sizeof(T) == 8;
+  ct::Args<T> g{};
+  g.na = (int)A.nstr;
+  g.nb = (int)B.nstr;
+  g.nbp = d->ct_nbp;
+  g.nsa = A.ns;
+  g.n = d->n;
+  g.mr = d->ct_mr;
+  g.R = d->ct_R;
+  g.kpad = d->ct_kpad;
+  g.seg_bytes = d->ct_seg;
+  g.part = A.nstr * d->ct_nbp;
+  g.a_sJ = (const int32_t*)A.sJ.ptr;
+  g.a_svo = (const int32_t*)A.svo.ptr;
+  g.rs_of = (const int32_t*)d->ct_rs.ptr;
+  g.seg = (const int32_t*)d->ct_segs.ptr;
+  g.a_sA = (const T*)(f64 ? A.sA64.ptr : A.sA32.ptr);
+  g.a_W = (const T*)(f64 ? A.W64.ptr : A.W32.ptr);
+  g.V2 = (const T*)(f64 ? d->ct_V64.ptr : d->ct_V32.ptr);
+  g.walk = (const uint16_t*)d->ct_walk.ptr;
+  g.Cs = (const uint16_t*)d->ct_C.ptr;
+  g.rexp = (const int*)d->ct_rexp.ptr;
+  g.D = (const double*)c->H.diag.ptr;
+  g.C = x;
+  g.sigma = y;
+  g.bad = (const int*)d->ct_flag.ptr + 1;
+  g.fault = d->ct_fault;
+  return g;
+}
+template <typename T>
+static void ct_launch(Context* c, const ct::Args<T>& g, int B) {
+  const ct::Smem<T> s(g.kpad, g.R, g.nb, g.seg_bytes);
+  auto go = [&](auto kern) {
+    set_max_dynamic_smem((const void*)kern, s.total);
+    kern<<<dim3((unsigned)g.na, (unsigned)B), (ct::Form<T>::EpiWarps + 1 + ct::kLoadWarps) * 32, s.total,
+           c->stream>>>(g);
+  };
+  switch (g.kpad / 16) {
+    case 1: go(ct::k_contract<T, 1>); break;
+    case 2: go(ct::k_contract<T, 2>); break;
+    case 3: go(ct::k_contract<T, 3>); break;
+    default: go(ct::k_contract<T, 4>); break;
+  }
+  QDKGB_CHECK_LAUNCH();
+}
+
+// y = sigma(x) in FP64 through the 16-bit digits: the dense same-spin
+// products, then the contraction with the diagonal.
+static void ct_sigma64(Context* c, const double* x, double* y) {
+  DirectSigma* d = c->direct;
+  const SpinTables& A = d->a;
+  const SpinTables& B = d->same ? d->a : d->b;
+  const int na = (int)A.nstr, nb = (int)B.nstr;
+  int* bad = (int*)d->ct_flag.ptr + 1;
+  int* rexp = (int*)d->ct_rexp.ptr;
+  int* cexp = (int*)d->ct_cexp.ptr;
+  QDKGB_CUDA(cudaMemsetAsync(bad, 0, 4, c->stream));
+  QDKGB_CUDA(cudaMemsetAsync(cexp, 0x80, (size_t)nb * 4, c->stream));
+  ct::Args<double> g = ct_args<double>(c, d, x, y);
+  ct::k_ct_split64<<<(unsigned)na, 256, 0, c->stream>>>(nb, d->ct_nbp, g.part, x, (uint16_t*)d->ct_C.ptr, rexp, bad);
+  QDKGB_CHECK_LAUNCH();
+  const int nkb1 = (na + ct::kDnK - 1) / ct::kDnK, nkb2 = (nb + ct::kDnK - 1) / ct::kDnK;
+  const int ta = (na + ct::kDnM - 1) / ct::kDnM, tb = (nb + ct::kDnN - 1) / ct::kDnN;
+  ct::k_dn_colexp<<<dim3((unsigned)((nb + 31) / 32), (unsigned)std::min(32, (na + 63) / 64)), 256, 0, c->stream>>>(
+      na, nb, x, cexp);
+  QDKGB_CHECK_LAUNCH();
+  ct::k_dn_split<<<dim3((unsigned)(tb * 2), (unsigned)(ta * 4)), 256, 0, c->stream>>>(
+      na, nb, x, rexp, cexp, nkb1, nkb2, ta * ct::kDnM, tb * ct::kDnN, (uint16_t*)d->dn_CA.ptr,
+      (uint16_t*)d->dn_CB.ptr);
+  QDKGB_CHECK_LAUNCH();
+  ct::DenseArgs q{na, nb, nkb1, nkb2, d->dn_flush, (const uint16_t*)d->dn_Ha.ptr, (const uint16_t*)d->dn_CB.ptr,
+                  (const uint16_t*)d->dn_CA.ptr, (const uint16_t*)d->dn_Hb.ptr, (const int*)d->dn_ea.ptr, cexp, rexp,
+                  (const int*)d->dn_eb.ptr, y, bad, g.fault};
+  ct::k_dense64<<<dim3((unsigned)tb, (unsigned)ta), ct::kDnThreads, ct::kDnStages * (ct::kDnA + ct::kDnB),
+                  c->stream>>>(q);
+  QDKGB_CHECK_LAUNCH();
+  ct_launch(c, g, 1);
+  ct::PlainArgs p{na,
+                  nb,
+                  d->n,
+                  A.ns,
+                  A.nd,
+                  B.ns,
+                  B.nd,
+                  (const int32_t*)A.sJ.ptr,
+                  (const int32_t*)A.svo.ptr,
+                  (const int32_t*)A.dJ.ptr,
+                  (const int32_t*)B.sJ.ptr,
+                  (const int32_t*)B.svo.ptr,
+                  (const int32_t*)B.dJ.ptr,
+                  (const double*)A.sA64.ptr,
+                  (const double*)A.dval64.ptr,
+                  (const double*)A.W64.ptr,
+                  (const double*)B.sA64.ptr,
+                  (const double*)B.dval64.ptr,
+                  (const double*)B.W64.ptr,
+                  (const double*)c->V.ptr,
+                  (const double*)c->H.diag.ptr,
+                  bad};
+  ct::k_plain64<<<(unsigned)na, 256, 0, c->stream>>>(p, x, y);
+  QDKGB_CHECK_LAUNCH();
+}
+
 // Values of every table from the current integrals (GPU).
 static void direct_values(Context* c, DirectSigma* d) {
   spin_values(c, d->a);
   if (!d->same) spin_values(c, d->b);
+  try {
+    ct_values(c, d);
+  } catch (const Error& e) {
+    // no memory for the 16-bit operands: the other forms serve
+    if (e.code != QDKGB_ERR_OOM) throw;
+    d->use32 = d->use64 = false;
+    for (DeviceBuffer* b : {&d->ct_C, &d->dn_Ha, &d->dn_Hb, &d->dn_CA, &d->dn_CB}) dev_free(c, *b);
+  }
   const int n = d->n;
   const int64_t n4 = (int64_t)n * n * n * n;
   float* V32 = dev_array<float>(c, d->V32, (size_t)n4);
@@ -1524,6 +1739,167 @@ static void build_mm_tables(Context* c, DirectSigma* d) {
   d->mm = true;
 }
 
+// Spaces from this many determinants up take the contraction from 16-bit
+// parts.  Measured, whole sigma, before -> after: FP32 12.9 thousand
+// determinants (9, 2, 5) 27 -> 31 us, 63.5 thousand (10, 5, 5) 48 -> 45 us,
+// 854 thousand (12, 6, 6) 366 -> 193 us; FP64 4.9 thousand 65 -> 71 us, 63.5
+// thousand 168 -> 126 us, 854 thousand 3.76 -> 0.72 ms.
+constexpr int64_t kCtMinDets = 32768;
+
+// Structure of the contraction from 16-bit parts (contract.cuh): the pair
+// rows, the walk lists; leaves d->ct false where it does not apply (more than
+// one 128-row tile, shared memory).  A chunk's list is 16-bit words: the bounds
+// of each warp's tasks (kHead words: of 16 warps, at word 32 of 8), the tasks'
+// order for 16 and for 8 warps (each padded to 8 words), four words per task
+// (offset of its entries / 32, steps, steps of the own-string rows, 0; padded
+// to 8 words), 32 target strings per task (0xffff: none), then the entries, 32
+// per step: the cell of E | sign << 15 (cell R kPitch is zero).  A task's 32
+// strings have similar step counts, so a warp's lanes stay busy; a string is
+// in one task of a chunk.
+static void build_ct_tables(Context* c, DirectSigma* d) {
+  d->ct = false;
+  const SpinTables& A = d->a;
+  const SpinTables& B = d->same ? d->a : d->b;
+  const int n = d->n;
+  const int64_t nb = B.nstr;
+  const int mr = n * (n - 1) / 2, R = mr + n + 1, kpad = (A.ns + 1 + 15) / 16 * 16;
+  if (A.nstr * nb < kCtMinDets) return;
+  if (A.ns <= 0 || B.ns <= 0 || B.h_packed.size() != (size_t)nb * B.ns || R > 128 || kpad > 64) return;
+  std::vector<int32_t> rmap((size_t)n * n, -1), rs_of(mr);
+  for (int q = 0, r = 0; q < n; ++q)
+    for (int p = 0; p < q; ++p) {
+      rmap[p + (size_t)n * q] = rmap[q + (size_t)n * p] = r;
+      rs_of[r++] = p + n * q;
+    }
+  const int nchunk = (int)((nb + ct::kCols - 1) / ct::kCols);
+  struct Item {
+    int ib, steps, own;
+  };
+  std::vector<std::vector<uint32_t>> ent((size_t)nchunk);  // ib << 16 | cell | sign << 15, by chunk
+  for (int64_t ib = 0; ib < nb; ++ib)
+    for (int l = 0; l < B.ns; ++l) {
+      const uint32_t w = B.h_packed[(size_t)ib * B.ns + l];
+      const uint32_t Jb = w & 0xffff, r = (uint32_t)rmap[(w >> 16) & 0x7fff];
+      ent[Jb / ct::kCols].push_back((uint32_t)ib << 16 | (r * ct::kPitch + Jb % ct::kCols) | (w >> 31) << 15);
+    }
+  std::vector<uint16_t> lists;
+  std::vector<int32_t> seg(nchunk + 1);
+  const uint16_t zero = (uint16_t)(R * ct::kPitch);
+  int seg_max = 0;
+  std::vector<int> first(nb + 1), cnt(nb);
+  for (int ch = 0; ch < nchunk; ++ch) {
+    seg[ch] = (int32_t)lists.size();
+    std::vector<uint32_t>& e = ent[ch];  // grouped by ib (pushed in ib order)
+    std::fill(cnt.begin(), cnt.end(), 0);
+    for (uint32_t w : e) ++cnt[w >> 16];
+    first[0] = 0;
+    for (int64_t ib = 0; ib < nb; ++ib) first[ib + 1] = first[ib] + cnt[ib];
+    std::vector<Item> items;
+    for (int64_t ib = 0; ib < nb; ++ib) {
+      const bool own = ib / ct::kCols == ch;
+      if (cnt[ib] || own) items.push_back({(int)ib, cnt[ib], own ? hpopc(c->dets.h_ubeta[ib]) + 1 : 0});
+    }
+    std::stable_sort(items.begin(), items.end(), [](const Item& x, const Item& y) {
+      return (x.own > 0) != (y.own > 0) ? x.own > 0 : x.steps > y.steps;
+    });
+    const int nt = (int)((items.size() + 31) / 32);
+    std::vector<uint16_t> head(ct::kHead, 0), order, task, tgt, body;
+    std::vector<int> cost;
+    for (int t = 0; t < nt; ++t) {
+      int steps = 0, own = 0;
+      const size_t i0 = (size_t)t * 32, i1 = std::min(items.size(), i0 + 32);
+      for (size_t i = i0; i < i1; ++i) {
+        steps = std::max(steps, items[i].steps);
+        own = std::max(own, items[i].own);
+      }
+      if (body.size() / 32 > 65535) return;
+      for (int v : {(int)(body.size() / 32), steps, own, 0}) task.push_back((uint16_t)v);
+      cost.push_back(steps + own + 6);  // about six steps' time goes to a task's start and end
+      const size_t b0 = body.size();
+      body.resize(b0 + (size_t)32 * (steps + own), zero);
+      for (int lane = 0; lane < 32; ++lane) {
+        if (i0 + lane >= i1) {
+          tgt.push_back(0xffff);
+          continue;
+        }
+        const Item& it = items[i0 + lane];
+        tgt.push_back((uint16_t)it.ib);
+        for (int s = 0; s < it.steps; ++s)
+          body[b0 + (size_t)32 * s + lane] = (uint16_t)(e[first[it.ib] + s] & 0xffff);
+        if (it.own) {
+          const uint64_t bits = c->dets.h_ubeta[it.ib];
+          int s = steps;
+          for (int p = 0; p < n; ++p)
+            if ((bits >> p) & 1)
+              body[b0 + (size_t)32 * s++ + lane] = (uint16_t)((mr + p) * ct::kPitch + it.ib % ct::kCols);
+          body[b0 + (size_t)32 * s + lane] = (uint16_t)((mr + n) * ct::kPitch + it.ib % ct::kCols);
+        }
+      }
+    }
+    if (task.size() % 8) task.resize(task.size() + 4, 0);
+    // the tasks over 16 and over 8 warps: longest first to the least loaded
+    for (int warps : {16, 8}) {
+      std::vector<int> by((size_t)nt), load(warps, 0);
+      for (int t = 0; t < nt; ++t) by[t] = t;
+      std::stable_sort(by.begin(), by.end(), [&](int x, int y) { return cost[x] > cost[y]; });
+      std::vector<std::vector<uint16_t>> mine(warps);
+      for (int t : by) {
+        const int w = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+        load[w] += cost[t];
+        mine[w].push_back((uint16_t)t);
+      }
+      const size_t o0 = order.size();
+      uint16_t* h = head.data() + (warps == 16 ? 0 : 32);
+      for (int w = 0; w < warps; ++w) {
+        h[w] = (uint16_t)(order.size() - o0);
+        order.insert(order.end(), mine[w].begin(), mine[w].end());
+      }
+      h[warps] = (uint16_t)nt;
+      order.resize(o0 + (size_t)((nt + 7) & ~7), 0);
+    }
+    for (const std::vector<uint16_t>* v : {&head, &order, &task, &tgt, &body}) lists.insert(lists.end(), v->begin(), v->end());
+    while (lists.size() % 8) lists.push_back(0);
+    seg_max = std::max(seg_max, (int)(lists.size() - seg[ch]));
+  }
+  seg[nchunk] = (int32_t)lists.size();
+  if (lists.size() >= (size_t)INT32_MAX) return;
+  if (ct::Smem<double>(kpad, R, (int)nb, seg_max * 2).total > 226 * 1024) return;
+  auto up = [&](DeviceBuffer& b, const void* src, size_t bytes) {
+    void* ptr = dev_alloc(c, b, bytes + 16);
+    QDKGB_CUDA(cudaMemcpyAsync(ptr, src, bytes, cudaMemcpyHostToDevice, c->stream));
+  };
+  up(d->ct_rs, rs_of.data(), rs_of.size() * 4);
+  up(d->ct_walk, lists.data(), lists.size() * 2);
+  up(d->ct_segs, seg.data(), seg.size() * 4);
+  d->ct_mr = mr;
+  d->ct_R = R;
+  d->ct_kpad = kpad;
+  d->ct_nbp = nchunk * ct::kCols;
+  d->ct_seg = seg_max * 2;
+  // the dense FP64 products' flush range: the most K blocks whose elements of
+  // any one row stay within kDnMaxRow
+  d->dn_flush = 0;
+  const int nkb = (int)((std::max(A.nstr, nb) + ct::kDnK - 1) / ct::kDnK);
+  for (int f = nkb; f >= 1; f = f > 1 ? (f + 1) / 2 : 0) {
+    int worst = 0;
+    for (const SpinTables* t : {&A, &B}) {
+      std::vector<int> h;
+      for (int64_t i = 0; i < t->nstr; ++i) {
+        h.assign((size_t)(t->nstr / (f * ct::kDnK)) + 1, 0);
+        for (int m = 0; m < t->nd; ++m) worst = std::max(worst, ++h[t->h_dJ[(size_t)i * t->nd + m] / (f * ct::kDnK)]);
+        for (int m = 0; m < t->ns; ++m)
+          worst = std::max(worst, ++h[(t->h_packed[(size_t)i * t->ns + m] & 0xffff) / (f * ct::kDnK)]);
+      }
+    }
+    if (worst <= ct::kDnMaxRow) {
+      d->dn_flush = f;
+      break;
+    }
+  }
+  QDKGB_CUDA(cudaStreamSynchronize(c->stream));
+  d->ct = true;
+}
+
 // The direct sigma's structure for the context's space (built once per
 // space; set_dets frees it) and its per-build settings from the environment.
 static DirectSigma* direct_structure(Context* c) {
@@ -1560,8 +1936,11 @@ static DirectSigma* direct_structure(Context* c) {
     // contraction form of the FP32 sigma, where its tables and shared memory
     // fit (QDKGB_DIRECT_MM=0 keeps the element-wise walk)
     build_mm_tables(c, d);
-    d->a.h_packed.clear();
-    d->b.h_packed.clear();
+    build_ct_tables(c, d);
+    for (SpinTables* t : {&d->a, &d->b}) {
+      t->h_packed.clear();
+      t->h_dJ.clear();
+    }
   }
   DirectSigma* d = c->direct;
   d->dense_env = dense_env;
@@ -1604,7 +1983,7 @@ static DirectSigma* direct_prepare(Context* c) {
 
 void direct_plan(const Context* c, int* mm, int* dense, double* ms) {
   const DirectSigma* d = c->direct;
-  if (mm) *mm = !(d && d->mm) ? 0 : (d->otc && d->otc_state == 1) ? 2 : 1;
+  if (mm) *mm = !(d && d->mm) ? 0 : (d->use32 || (d->otc && d->otc_state == 1)) ? 2 : 1;
   if (dense) *dense = d ? d->dense_state : -1;
   if (ms) {
     ms[0] = d ? d->dense_ms[0] : 0.;
@@ -1627,9 +2006,33 @@ bool attach_direct_fp32(Context* c) {
   return d->mm;
 }
 
+// Stored complete spaces from this size up take their FP64 sigma through the
+// 16-bit digits as well (the matrix stays for the exports): 854 thousand
+// determinants 2.82 ms from the slab, 0.72 ms; 63.5 thousand 138 and 126 us,
+// where the tables' set-up (0.3 ms and more on the host) would not pay.
+constexpr int64_t kCtStoredMinDets = (int64_t)1 << 17;
+
+bool attach_direct_fp64(Context* c, double thresh, bool prepared) {
+  // the digits hold every element: only where the threshold is no more than
+  // the rounding of the largest ones
+  if (c->dets.ndets < kCtStoredMinDets || thresh > std::numeric_limits<double>::epsilon()) return false;
+  size_t fr = 0, tot = 0;
+  QDKGB_CUDA(cudaMemGetInfo(&fr, &tot));
+  // beside a Davidson workspace of any size
+  if ((double)fr < (double)c->dets.ndets * (8.0 * 530 + 128)) return false;
+  DirectSigma* d = c->direct;
+  try {
+    if (!prepared) d = direct_prepare(c);
+  } catch (const Error& e) {
+    if (e.code == QDKGB_ERR_CUDA) throw;
+    return false;
+  }
+  return d->use64;
+}
+
 void build_direct_sigma(Context* c) {
   NvtxRange nvtx_range("qdkgb.build_direct_sigma");
-  c->fp32_direct = false;
+  c->fp32_direct = c->fp64_direct = false;
   direct_prepare(c);
   DetSpace& S = c->dets;
   // diagonal and operator state

@@ -148,6 +148,8 @@ struct Context {
   bool op_direct = false;         // Davidson / spmv use the direct sigma instead of the CSR
   bool fp32_direct = false;       // complete space, mixed form: FP32 sigma by the direct contraction,
                                   // full-precision sigma by the stored (FP64) slab
+  bool fp64_direct = false;       // stored complete space whose FP64 sigma runs through the direct
+                                  // contraction's 16-bit digits
   // seconds spent by the last qdkgb_asci call in its phases: the determinant
   // search, the determinant-space set-up, the Hamiltonian build, Davidson;
   // and its asci_iter count
@@ -258,6 +260,11 @@ void build_direct_sigma(Context* c);
 // the stored FP64 slab (mixed form); false where the contraction form does
 // not apply.
 bool attach_direct_fp32(Context* c);
+// The FP64 sigma of a stored complete space through the direct contraction's
+// 16-bit digits; false where that form does not apply (small spaces, a
+// threshold above the machine epsilon, integrals without V(..|rs) = V(..|sr)).
+// prepared: attach_direct_fp32 has just made the tables.
+bool attach_direct_fp64(Context* c, double thresh, bool prepared);
 // Batched CASCI's FP32 sigma through the direct contraction: per-instance
 // value tables of a sub-batch (T: [B][n^2], V: [B][n^4] on the device; false
 // where the form does not apply), then y = sigma(x) for the active instances

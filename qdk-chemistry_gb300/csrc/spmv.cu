@@ -131,7 +131,7 @@ static unsigned spmv_blocks(Context* c, int64_t n) {
 void spmv_fp64(Context* c, const double* x, double* y) {
   Hcsr& H = c->H;
   if (!H.valid) throw Error(QDKGB_ERR_STATE, "Hamiltonian not built");
-  if (c->op_direct) {
+  if (c->op_direct || c->fp64_direct) {
     direct_sigma_fp64(c, x, y);
     return;
   }
