@@ -864,7 +864,7 @@ double sci_diag_gpu(Context* c, const qdkgb_asci_settings& S, const qdkgb_davids
   X.resize(n, 0.);
   if (!s.use_guess) std::fill(X.begin(), X.end(), 0.);
   double E = 0.;
-  davidson(c, &s, &E, X.data(), nullptr);
+  davidson(c, &s, &E, X.data(), nullptr, true);
   clock.lap(3);
   return E;
 }

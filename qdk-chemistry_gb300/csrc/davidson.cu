@@ -763,8 +763,15 @@ __global__ void __launch_bounds__(kFlipTile * 8) k_df_flip_project(float2* x, in
 }
 
 __global__ void __launch_bounds__(kEigThreads) k_lowest_eig(int k, const double* __restrict__ H, int ldh,
-                                                            double* gA, int nev, double* eval, double* evec) {
-  lowest_eig_cta(k, H, ldh, gA, nev, eval, evec);
+                                                            double* gA, int nev, double* eval, double* evec,
+                                                            bool keep0) {
+  lowest_eig_cta(k, H, ldh, gA, nev, eval, evec, nullptr, keep0);
+}
+// the lowest pair of a matrix that grew by one row since the last call on st
+__global__ void __launch_bounds__(kEigThreads) k_lowest_eig_next(int k, const double* __restrict__ H, int ldh,
+                                                                 double* gA, double* eval, double* evec,
+                                                                 EigWarm* st) {
+  lowest_eig_next_cta(k, H, ldh, gA, eval, evec, st);
 }
 
 // One CTA per instance of a batch: the lowest pair of the leading k x k block
@@ -810,6 +817,7 @@ struct Dav {
   int nb;  // blocks of the row-parallel kernels (partial sums per column)
   int sm_count;
   double* gA = nullptr;
+  EigWarm* warm = nullptr;  // the projected problem's state from size to size
   cudaStream_t st;
 
   unsigned* counts() { return (unsigned*)(small + kSlotCount); }
@@ -898,11 +906,22 @@ struct Dav {
   }
 
   // lowest `nev` eigenpairs of the leading k x k projected matrix
-  void lowest(int k, int nev = 1) {
+  void lowest(int k, int nev = 1, bool keep0 = false) {
     const bool in_smem = k <= kEigSmemK;
+    if (nev == 1 && warm) {
+      const size_t dyn = std::max(in_smem ? eig_dyn_smem(k) : (size_t)0, k <= kEigWarmMaxK ? eig_warm_smem(k) : (size_t)0);
+      k_lowest_eig_next<<<1, kEigThreads, dyn, st>>>(k, Hk, (int)(maxm + 1), in_smem ? nullptr : gA, eval, evec, warm);
+      QDKGB_CHECK_LAUNCH();
+      return;
+    }
     k_lowest_eig<<<1, kEigThreads, in_smem ? eig_dyn_smem(k) : 0, st>>>(
-        k, Hk, (int)(maxm + 1), in_smem ? nullptr : gA, std::min(nev, k), eval, evec);
+        k, Hk, (int)(maxm + 1), in_smem ? nullptr : gA, std::min(nev, k), eval, evec, keep0);
     QDKGB_CHECK_LAUNCH();
+  }
+
+  // the projected matrix is another one from here on
+  void forget_warm() {
+    if (warm) QDKGB_CUDA(cudaMemsetAsync(warm, 0, 8, st));
   }
 
   // new row i of the projected matrix, Hk(i, c) = V_i . AV_c for c <= i,
@@ -1087,7 +1106,7 @@ static void davidson_roots(Context* c, const qdkgb_davidson_settings* s, double*
     out = h;
   };
   auto lowest_fp64 = [&](int k) {
-    k_lowest_eig<<<1, kEigThreads, 0, d.st>>>(k, d.Hk, (int)(max_m + 1), d.gA, R, d.eval, d.evec);
+    k_lowest_eig<<<1, kEigThreads, 0, d.st>>>(k, d.Hk, (int)(max_m + 1), d.gA, R, d.eval, d.evec, false);
     QDKGB_CHECK_LAUNCH();
   };
   // append w (already in V[:, k]) : orthonormalise, sigma, projected row
@@ -1174,7 +1193,8 @@ static void davidson_roots(Context* c, const qdkgb_davidson_settings* s, double*
   if (!converged) throw Error(QDKGB_ERR_NOT_CONVERGED, "Davidson Did Not Converge!");
 }
 
-void davidson(Context* c, const qdkgb_davidson_settings* s, double* E, double* C, qdkgb_davidson_info* info) {
+void davidson(Context* c, const qdkgb_davidson_settings* s, double* E, double* C, qdkgb_davidson_info* info,
+              bool steady) {
   if (s->nroots > 1) {
     if (!c->H.valid) throw Error(QDKGB_ERR_STATE, "Hamiltonian not built");
     davidson_roots(c, s, E, C, info);
@@ -1216,6 +1236,13 @@ void davidson(Context* c, const qdkgb_davidson_settings* s, double* E, double* C
   d.small = dev_array<double>(c, W.small, 4 * kMaxSubspace);
   if (max_m + 1 > kEigSmemK) d.gA = dev_array<double>(c, W.yf, (size_t)(max_m + 1) * (max_m + 1));
   set_max_dynamic_smem((const void*)k_lowest_eig, (int)kEigDynSmemMax);
+  set_max_dynamic_smem((const void*)k_lowest_eig_next, (int)kEigDynSmemMax);
+  try {
+    if (!steady) d.warm = dev_array<EigWarm>(c, W.eig, 1);
+  } catch (const Error& e) {
+    if (e.code != QDKGB_ERR_OOM) throw;  // at a memory cap: every size from scratch
+  }
+  d.forget_warm();
   d.D = (double*)H.diag.ptr;
   d.clear_flag();
   QDKGB_CUDA(cudaMemsetAsync(d.counts(), 0, (kDotChunks + 1) * sizeof(unsigned), c->stream));
@@ -1287,6 +1314,7 @@ void davidson(Context* c, const qdkgb_davidson_settings* s, double* E, double* C
       if (degenerate) {
         // V[:, i] was not normalisable: repair it and redo this iteration
         d.fallback((int)i, d.col(d.V, i));
+        d.forget_warm();
         --i;
         --iter;
         continue;
@@ -1398,6 +1426,7 @@ void davidson(Context* c, const qdkgb_davidson_settings* s, double* E, double* C
         --k;
         --iter;
         d.df_fallback(k, d.colf(d.Vf, k));
+        d.forget_warm();
         continue;
       }
       const double est = std::sqrt(r2);
@@ -1434,7 +1463,7 @@ void davidson(Context* c, const qdkgb_davidson_settings* s, double* E, double* C
       }
       // thick restart: V' = V Q[:, 0:kk], AV' = AV Q[:, 0:kk]; column 0 = X with its exact sigma
       const int kk = std::min(kKeep, k);
-      d.lowest(k, kk);  // the kk lowest Ritz vectors (column 0 reproduces X)
+      d.lowest(k, kk, true);  // the kk lowest Ritz vectors (column 0 reproduces X)
       if (kk > 1) {
         static_assert(kKeep - 1 <= kMaxOut, "restart block wider than k_df_gemv_multi");
         k_df_gemv_multi<<<d.nb, kVecThreads, 0, c->stream>>>(d.Vf, N, k, d.evec + k, kk - 1, tmpV, N, N);
@@ -1451,6 +1480,7 @@ void davidson(Context* c, const qdkgb_davidson_settings* s, double* E, double* C
                                    cudaMemcpyDeviceToDevice, c->stream));
       }
       for (int j = 0; j < kk; ++j) d.df_projected_row(j);
+      d.forget_warm();
       k = kk;
       // next direction: preconditioned true residual
       k_precondition<<<d.nb, 256, 0, c->stream>>>(Rt, d.D, Eptr, N, s->min_abs_denominator);

@@ -114,7 +114,7 @@ struct Hcsr {
 };
 
 struct DavidsonWork {
-  DeviceBuffer V, AV, xf, yf, Hk, evec, eval, scratch, partial, small;
+  DeviceBuffer V, AV, xf, yf, Hk, evec, eval, scratch, partial, small, eig;
   int64_t n = 0, maxm = 0;
 };
 
@@ -292,8 +292,13 @@ void asci_run(Context* c, const qdkgb_asci_settings& S, const qdkgb_davidson_set
               std::vector<uint64_t>& a, std::vector<uint64_t>& b, std::vector<double>& X, double& E0, bool grow,
               bool refine, double* E_grow);
 
-// davidson.cu
-void davidson(Context* c, const qdkgb_davidson_settings* s, double* E, double* C, qdkgb_davidson_info* info);
+// davidson.cu.  steady: the projected problem is solved from scratch at every
+// size instead of from the size before, for callers whose further course hangs
+// on the last bits of the vector: an ASCI grow cuts its lists by |C| and |rv|,
+// where a determinant and its spin-flip twin differ by rounding alone, so that
+// another rounding picks other twins.
+void davidson(Context* c, const qdkgb_davidson_settings* s, double* E, double* C, qdkgb_davidson_info* info,
+              bool steady = false);
 
 // rdm.cu
 void rdms_spin_dep(Context* c, const double* C, double* aa, double* bb, double* aaaa, double* bbbb, double* aabb);

@@ -62,21 +62,35 @@ static __device__ int sturm_count(int k, const double* d, const double* e2, doub
   return cnt;
 }
 
+struct EigWarm;
 static __device__ bool lowest_eig_mixed_cta(int k, const double* __restrict__ H, int ldh, int nev, double* eval,
-                                     double* evec, unsigned char* smem);
+                                     double* evec, unsigned char* smem, EigWarm* st, bool keep0);
 constexpr int kEigMixedMaxK = 128;
 
+// What one projected problem leaves for the next, which is the same matrix
+// with one more row (lowest_eig_warm_cta): P = (H - sigma)^-1 of the leading k
+// x k block in FP32, sigma below its lowest eigenvalue, and the lowest pair.
+// k = 0: none.  kt: the size theta belongs to.
+constexpr int kEigWarmMaxK = 220;  // P in shared memory
+struct EigWarm {
+  int k, kt;
+  double sigma, theta, scale, gap;  // gap: to the next eigenvalue, when P was made
+  double x[kEigWarmMaxK];
+  float P[kEigWarmMaxK * kEigWarmMaxK];  // leading dimension k
+};
+
 static __device__ void lowest_eig_cta(int k, const double* __restrict__ H, int ldh, double* gA, int nev, double* eval,
-                               double* evec) {
+                               double* evec, EigWarm* st = nullptr, bool keep0 = false) {
   extern __shared__ double dyn[];
   __shared__ double d[kEigMaxK], e[kEigMaxK], e2[kEigMaxK], beta[kEigMaxK];
   __shared__ double red[33];
   __shared__ double s_lo, s_hi;
   __shared__ double s_u[3 * kEigMaxK];
   if (nev >= 1 && nev <= k && k >= 2 && k <= kEigMixedMaxK && !gA) {
-    if (lowest_eig_mixed_cta(k, H, ldh, nev, eval, evec, reinterpret_cast<unsigned char*>(dyn))) return;
+    if (lowest_eig_mixed_cta(k, H, ldh, nev, eval, evec, reinterpret_cast<unsigned char*>(dyn), st, keep0)) return;
     __syncthreads();
   }
+  if (st && threadIdx.x == 0) st->k = st->kt = 0;
   double* A = gA ? gA : dyn;  // k x k, column-major; reflector j kept in column j below the diagonal
   const int tid = threadIdx.x, nt = blockDim.x;
   for (int t = tid; t < k * k; t += nt) {
@@ -280,6 +294,11 @@ namespace qdkgb {
 // products.  Returns false (the caller takes the FP64 path) for a
 // near-degenerate lowest pair or when the refinement does not reach rounding
 // level.
+// keep0: evec[:, 0] holds the lowest eigenvector of this matrix already (the
+// solve before): it stays as it is, and the further columns are made
+// orthogonal to it (a thick restart keeps the Ritz vector formed from it; two
+// solves' vectors differ by rounding over the gap, which the restarted basis
+// would carry as an overlap).
 
 // sum over aligned groups of g lanes (g a power of two <= 32); every lane of
 // the warp takes part
@@ -295,7 +314,7 @@ __device__ __forceinline__ T group_sum(T v, int g) {
 // component r of eigenvector i, ldq = k | 1), d, e, e2, beta, lam, lamhi, vec
 // (kEigMixedMaxK each), red[32]
 static __device__ bool lowest_eig_mixed_cta(int k, const double* __restrict__ H, int ldh, int nev, double* eval,
-                                     double* evec, unsigned char* smem) {
+                                     double* evec, unsigned char* smem, EigWarm* st, bool keep0) {
   const int tid = threadIdx.x, nt = blockDim.x;
   const int wid = tid >> 5, lane = tid & 31;
   const int ldq = k | 1;
@@ -503,11 +522,13 @@ static __device__ bool lowest_eig_mixed_cta(int k, const double* __restrict__ H,
   // theta = y.w / y.y, |r| / |y|.  Every warp forms the same sums in the same
   // order, so theta and |r| are known everywhere without a barrier.
   for (int t = tid; t < k * k; t += nt) R[t] = Hat(t % k, t / k);
-  for (int i = tid; i < k; i += nt) y[i] = (double)Q[i * ldq];
+  for (int i = tid; i < k; i += nt) y[i] = keep0 ? evec[i] : (double)Q[i * ldq];
   __syncthreads();
   const double eps = 1.1102230246251565e-16, hs = (double)scale + 1e-300;
   double theta = 0., rn = 1e300, rprev = 1e300;
+  int it0 = 0;
   for (int it = 0; it < 8; ++it) {
+    it0 = it;
     double acc = 0.;
     if (gc < k)
       for (int l = gs; l < k; l += g) acc += R[l + (size_t)k * gc] * y[l];
@@ -528,7 +549,7 @@ static __device__ bool lowest_eig_mixed_cta(int k, const double* __restrict__ H,
       rr += ri * ri;
     }
     rn = sqrt(warp_sum(rr) / yy);
-    if (rn <= 16. * eps * hs || (it >= 2 && rn > 0.5 * rprev)) break;
+    if (rn <= (keep0 ? 128. : 16.) * eps * hs || (it >= 2 && rn > 0.5 * rprev)) break;
     rprev = rn;
     // c_i = q_i . r / (l_i - theta), i > 0 (FP32), group gc = i
     float c = 0.f;
@@ -546,7 +567,7 @@ static __device__ bool lowest_eig_mixed_cta(int k, const double* __restrict__ H,
     __syncthreads();
   }
   if (!(rn <= 4096. * eps * hs)) return false;
-  {
+  if (!(keep0 && it0 == 0)) {
     double yy = 0.;
     for (int i = lane; i < k; i += 32) yy += y[i] * y[i];
     const double inv = 1. / sqrt(warp_sum(yy));
@@ -554,6 +575,36 @@ static __device__ bool lowest_eig_mixed_cta(int k, const double* __restrict__ H,
   }
   if (tid == 0) eval[0] = theta;
   __syncthreads();
+  if (st) {
+    // the inverse for the next size: a shift four times the last drop of the
+    // lowest eigenvalue below it (the drops of a converging iteration fall
+    // geometrically), none while that is a large part of the gap
+    const double gap = (double)(lam[1] - lam[0]), dec = st->kt == k - 1 ? st->theta - theta : 1e300;
+    const double delta = fmax(4. * dec, 1e-3 * gap);
+    const bool build = nev == 1 && delta <= 0.2 * gap;
+    __syncthreads();
+    if (tid == 0) {
+      st->k = build ? k : 0;
+      st->kt = k;
+      st->theta = theta;
+      st->sigma = theta - delta;
+      st->scale = hs;
+      st->gap = gap;
+    }
+    if (build) {
+      for (int i = tid; i < k; i += nt) {
+        st->x[i] = evec[i];
+        vec[i] = i ? 1.f / (lam[i] - (float)(theta - delta)) : (float)(1. / delta);
+      }
+      __syncthreads();
+      for (int t = tid; t < k * k; t += nt) {
+        const int i = t % k, j = t / k;
+        float p = 0.f;
+        for (int m = 0; m < k; ++m) p += Q[i * ldq + m] * vec[m] * Q[j * ldq + m];
+        st->P[t] = p;
+      }
+    }
+  }
   if (nev == 1) return true;
   // Further columns (a thick-restart basis): the FP32 eigenvectors 1..nev-1,
   // orthonormalised in FP64 against the columns before them (classical
@@ -588,6 +639,213 @@ static __device__ bool lowest_eig_mixed_cta(int k, const double* __restrict__ H,
   return s_ok != 0;
 }
 
+// shared-memory bytes of lowest_eig_warm_cta: P, the matrix where it is kept
+// there (k <= kEigMixedMaxK), partial sums and vectors
+__host__ __device__ constexpr size_t eig_warm_smem(int k) {
+  return (size_t)((k * k + 1) & ~1) * sizeof(float) +
+         ((size_t)(k <= kEigMixedMaxK ? k * k : 0) + 8 * 32 + 256 + 3 * (size_t)kEigWarmMaxK) * sizeof(double);
+}
+
+// The lowest pair of the k x k matrix H (full, symmetric) whose leading (k -
+// 1)-block was solved before (st).  P is bordered for the new row (a rank-one
+// update), then y <- y - z, z ~ (H - theta)^-1 r off y, r = H y - theta y in
+// FP64, from y = the last vector.  (H - theta)^-1 = P + delta P^2 + delta^2 P^3
+// .., delta = theta - sigma: each further term costs one FP32 product and
+// shortens the error by delta / (delta + gap), so that two or three FP64
+// products reach rounding level, where the full solve's reflectors,
+// bisections and back-transforms are k-long chains.
+// Returns false (the full solve follows) when sigma is no longer below the
+// spectrum or the steps do not reach rounding level.
+static __device__ bool lowest_eig_warm_cta(int k, const double* __restrict__ H, int ldh, double* eval, double* evec,
+                                           unsigned char* smem, EigWarm* st) {
+  const int tid = threadIdx.x, lane = tid & 31, k1 = k - 1;
+  const int kr = (k + 31) & ~31, parts = kEigThreads / kr, row = tid % kr, part = tid / kr;
+  const bool in_smem = k <= kEigMixedMaxK;
+  double* y = reinterpret_cast<double*>(smem);
+  double* w = y + kEigWarmMaxK;
+  double* b = w + kEigWarmMaxK;
+  double* ps = b + kEigWarmMaxK;  // [parts][kr], at most 256 + 8 * 32
+  double* R = ps + 8 * 32 + 256;
+  float* P = reinterpret_cast<float*>(R + (in_smem ? k * k : 0));
+  float* v = reinterpret_cast<float*>(w);   // FP32 operand of P
+  float* pf = reinterpret_cast<float*>(ps);
+  const double sigma = st->sigma, hs = st->scale;
+  if (in_smem)
+    for (int t = tid; t < k * k; t += kEigThreads) R[t] = H[t % k + (size_t)(t / k) * ldh];
+  for (int t = tid; t < k1 * k1; t += kEigThreads) P[t % k1 + k * (t / k1)] = st->P[t];
+  for (int i = tid; i < k; i += kEigThreads) {
+    y[i] = i < k1 ? st->x[i] : 0.;
+    b[i] = H[i + (size_t)k1 * ldh];
+    v[i] = (float)b[i];
+  }
+  __syncthreads();
+  // M u for a column-major M: a thread per row and column part
+  auto times_P = [&](int m) {
+    float a = 0.f;
+    if (part < parts && row < m)
+      for (int l = part; l < m; l += parts) a += P[row + k * l] * v[l];
+    if (part < parts) pf[part * kr + row] = a;
+  };
+  auto sum_f = [&](int i) {
+    float a = 0.f;
+    for (int q = 0; q < parts; ++q) a += pf[q * kr + i];
+    return a;
+  };
+  times_P(k1);
+  __syncthreads();
+  double bg = 0.;
+  for (int i = lane; i < k1; i += 32) bg += b[i] * (double)sum_f(i);
+  bg = warp_sum(bg);
+  const double s = (b[k1] - sigma) - bg;
+  if (!(s > 1e-6 * hs)) return false;  // the same in every thread
+  const float si = (float)(1. / s);
+  __syncthreads();
+  for (int i = tid; i < k1; i += kEigThreads) v[i] = sum_f(i);
+  __syncthreads();
+  for (int t = tid; t < k * k; t += kEigThreads) {
+    const int i = t % k, j = t / k;
+    if (i < k1 && j < k1)
+      P[t] += v[i] * v[j] * si;
+    else
+      P[t] = i < k1 ? -v[i] * si : j < k1 ? -v[j] * si : si;
+    st->P[t] = P[t];
+  }
+  __syncthreads();
+  // One warp does the vector work of a step (the FP64 pipe, two lanes a
+  // clock for the whole SM, is what eight warps forming the same sums would
+  // wait for); the others take part in the products.
+  __shared__ int s_state;  // 0: go on, 1: at rounding level, 2: given up
+  __shared__ int s_terms;
+  const double eps = 1.1102230246251565e-16;
+  const double fine = 16. * eps * hs, coarse = 64. * eps * hs;
+  constexpr int kSteps = 10, kQ = (kEigWarmMaxK + 31) / 32;
+  const int dparts = min(parts, 4);
+  double theta = 0., yy = 1., rprev = 1e300;
+  float delta = 0.f, iyy = 1.f;
+  int it = 0;
+  for (;; ++it) {
+    if (part < dparts && row < k) {
+      double a = 0.;
+      if (in_smem) {
+        for (int l = part; l < k; l += dparts) a += R[row + k * l] * y[l];
+      } else {
+#pragma unroll 8
+        for (int l = part; l < k; l += dparts) a += __ldg(H + row + (size_t)l * ldh) * y[l];
+      }
+      ps[part * kr + row] = a;
+    }
+    __syncthreads();
+    float yf[kQ], z0[kQ];
+    if (tid < 32) {
+      double hw[kQ], yw = 0., rr = 0.;
+      yy = 0.;
+#pragma unroll
+      for (int q = 0; q < kQ; ++q) {
+        const int i = lane + 32 * q;
+        if (32 * q >= k) break;
+        hw[q] = 0.;
+        if (i < k) {
+          for (int p = 0; p < dparts; ++p) hw[q] += ps[p * kr + i];
+          yy += y[i] * y[i];
+          yw += y[i] * hw[q];
+        }
+      }
+      yy = warp_sum(yy);
+      yw = warp_sum(yw);
+      theta = yw / yy;
+#pragma unroll
+      for (int q = 0; q < kQ; ++q) {
+        const int i = lane + 32 * q;
+        if (32 * q >= k) break;
+        if (i < k) {
+          const double ri = hw[q] - theta * y[i];
+          rr += ri * ri;
+          v[i] = (float)ri;
+          yf[q] = (float)y[i];
+        }
+      }
+      rr = warp_sum(rr);  // |r|^2 |y|^2: against the levels times |y|^2
+      const bool small = rr <= coarse * coarse * yy;
+      int state = 0;
+      if (rr <= fine * fine * yy)
+        state = 1;
+      else if (it >= 2 && rr > 0.25 * rprev)
+        state = small ? 1 : 2;
+      else if (it + 1 == kSteps)
+        state = small ? 1 : 2;
+      rprev = rr;
+      delta = (float)(theta - sigma);
+      iyy = 1.f / (float)yy;
+      if (lane == 0) {
+        const float f = delta / (delta + (float)st->gap);
+        s_state = state;
+        s_terms = f > 0.f ? min(6, (int)ceilf(-13.8f / __logf(fminf(f, 0.9f)))) : 1;
+      }
+    }
+    __syncthreads();
+    if (s_state) break;
+    const int terms = s_terms;
+    for (int t = 0; t < terms; ++t) {
+      times_P(k);
+      __syncthreads();
+      if (tid < 32) {
+        // z <- z0 + delta P z off y (z0 = P r off y first)
+        float z[kQ], yt = 0.f;
+#pragma unroll
+        for (int q = 0; q < kQ; ++q) {
+          const int i = lane + 32 * q;
+          if (32 * q >= k) break;
+          z[q] = i < k ? sum_f(i) : 0.f;
+          if (i < k) yt += yf[q] * z[q];
+        }
+        yt = warp_sum(yt) * iyy;
+#pragma unroll
+        for (int q = 0; q < kQ; ++q) {
+          const int i = lane + 32 * q;
+          if (32 * q >= k) break;
+          if (i < k) {
+            float x = z[q] - yt * yf[q];
+            if (t == 0)
+              z0[q] = x;
+            else
+              x = z0[q] + delta * x;
+            v[i] = x;
+            if (t == terms - 1) y[i] -= (double)x;
+          }
+        }
+      }
+      __syncthreads();
+    }
+  }
+  if (s_state == 2) return false;
+  if (tid < 32) {
+    const double inv = 1. / sqrt(yy);
+    for (int i = lane; i < k; i += 32) {
+      const double xi = y[i] * inv;
+      evec[i] = xi;
+      st->x[i] = xi;
+    }
+  }
+  if (tid == 0) {
+    eval[0] = theta;
+    // many steps: sigma is far below by now, the next solve makes a new P
+    st->k = it >= 7 && k < kEigMixedMaxK ? 0 : k;
+    st->kt = k;
+    st->theta = theta;
+  }
+  return true;
+}
+
+// The lowest pair with the state of the size before, where it serves
+static __device__ void lowest_eig_next_cta(int k, const double* __restrict__ H, int ldh, double* gA, double* eval,
+                                           double* evec, EigWarm* st) {
+  extern __shared__ double dyn[];
+  const bool warm = k >= 3 && k <= kEigWarmMaxK && st->k == k - 1;
+  if (warm && lowest_eig_warm_cta(k, H, ldh, eval, evec, reinterpret_cast<unsigned char*>(dyn), st)) return;
+  __syncthreads();
+  lowest_eig_cta(k, H, ldh, gA, 1, eval, evec, st);
+}
+
 // shared-memory bytes of lowest_eig_mixed_cta for size k
 __host__ __device__ constexpr size_t eig_mixed_smem(int k) {
   return (2 * (size_t)kEigMixedMaxK + (size_t)k * k) * sizeof(double) +
@@ -602,8 +860,9 @@ __host__ __device__ constexpr size_t eig_dyn_smem(int k) {
 
 // the largest dynamic shared memory lowest_eig_cta asks for (matrices up to
 // kEigSmemK in shared memory)
-constexpr size_t kEigDynSmemMax = eig_mixed_smem(kEigMixedMaxK) > (size_t)kEigSmemK * kEigSmemK * sizeof(double)
-                                      ? eig_mixed_smem(kEigMixedMaxK)
-                                      : (size_t)kEigSmemK * kEigSmemK * sizeof(double);
+constexpr size_t eig_max(size_t a, size_t b) { return a > b ? a : b; }
+constexpr size_t kEigDynSmemMax =
+    eig_max(eig_max(eig_mixed_smem(kEigMixedMaxK), (size_t)kEigSmemK * kEigSmemK * sizeof(double)),
+            eig_max(eig_warm_smem(kEigMixedMaxK), eig_warm_smem(kEigWarmMaxK)));
 
 }  // namespace qdkgb
