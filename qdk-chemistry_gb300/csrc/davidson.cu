@@ -55,6 +55,33 @@ __device__ __forceinline__ double block_sum_vec(double v, double* red) {
   return t;
 }
 
+// Sums of eight values per lane over the warp: lane l returns the sum of
+// v[(l >> 4 & 1) * 4 + (l >> 3 & 1) * 2 + (l >> 2 & 1)].  The halves of the
+// butterfly exchange columns as they add, nine additions instead of forty,
+// each sum over the same tree as warp_sum (the same value bit for bit).  The
+// forty were most of a small product: an FP64 addition of a warp holds the
+// SM's two-lane FP64 pipe for sixteen clocks.
+template <typename T, typename Add, typename Shfl>
+__device__ __forceinline__ T warp_sum8(T* v, Add add, Shfl shfl) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int h = 4; h >= 1; h >>= 1) {
+    const int d = 4 * h;
+    const bool up = lane & d;
+#pragma unroll
+    for (int q = 0; q < h; ++q) {
+      const T other = shfl(up ? v[q] : v[q + h], d);
+      v[q] = add(up ? v[q + h] : v[q], other);
+    }
+  }
+  v[0] = add(v[0], shfl(v[0], 2));
+  return add(v[0], shfl(v[0], 1));
+}
+__device__ __forceinline__ int warp_sum8_col() {
+  const int lane = threadIdx.x & 31;
+  return ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+}
+
 // Called by every thread after this block stored its partial sums: true in
 // the block that finished last (count[slot] is then reset for the next
 // launch).  Its reads of the other blocks' partials go through L2 (__ldcg).
@@ -71,6 +98,52 @@ __device__ __forceinline__ bool last_block_done(unsigned* count, int slot, unsig
   return last;
 }
 
+// The end of k_multidot and k_df_multidot: this block's column sums (red: per
+// warp), its partial sums, and in the last block the totals.  With Hk the
+// totals also are row hrow of the projected matrix, Hk(hrow, c) = Hk(c, hrow)
+// (syev reads the lower triangle, rayleigh_ritz.hpp:70-77; the warm
+// eigensolve the whole).
+__device__ __forceinline__ void dot_finish(double (*red)[kDotCols + 1], int j0, int nc, int k, bool self,
+                                           double* __restrict__ partial, unsigned* __restrict__ count,
+                                           double* __restrict__ out, int out_stride, double* __restrict__ self_out,
+                                           int hrow, double* __restrict__ Hk, int ldh) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  __syncthreads();
+  if (threadIdx.x < nc) {
+    double t = 0.;
+    for (int q = 0; q < kVecThreads / 32; ++q) t += red[q][threadIdx.x];
+    partial[(size_t)(j0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
+  }
+  if (self && threadIdx.x == kDotCols) {
+    double t = 0.;
+    for (int q = 0; q < kVecThreads / 32; ++q) t += red[q][kDotCols];
+    partial[(size_t)k * gridDim.x + blockIdx.x] = t;
+  }
+  if (!last_block_done(count, blockIdx.y, gridDim.x)) return;
+  if (wid < nc) {
+    const int j = j0 + wid;
+    const double* p = partial + (size_t)j * gridDim.x;
+    double t = 0.;
+    for (int b = lane; b < (int)gridDim.x; b += 32) t += __ldcg(p + b);
+    t = warp_sum(t);
+    if (lane == 0) {
+      if (Hk) {
+        Hk[hrow + (size_t)j * ldh] = t;
+        Hk[j + (size_t)hrow * ldh] = t;
+      } else {
+        out[(size_t)j * out_stride] = t;
+      }
+    }
+  }
+  if (self && wid == kVecThreads / 32 - 1) {
+    const double* p = partial + (size_t)k * gridDim.x;
+    double t = 0.;
+    for (int b = lane; b < (int)gridDim.x; b += 32) t += __ldcg(p + b);
+    t = warp_sum(t);
+    if (lane == 0) *self_out = t;
+  }
+}
+
 // out[j * out_stride] = A[:, j] . w for j < k.  Block (x, y) takes columns
 // y*kDotCols .. +kDotCols over a grid-stride share of the rows, so w is read
 // once per column block; partial sums go to partial[j * gridDim.x + x] and the
@@ -81,7 +154,8 @@ __device__ __forceinline__ bool last_block_done(unsigned* count, int slot, unsig
 __global__ void __launch_bounds__(kVecThreads)
     k_multidot(const double* __restrict__ A, int64_t lda, int k, const double* __restrict__ w, int64_t n,
                double* __restrict__ partial, unsigned* __restrict__ count, double* __restrict__ out, int out_stride,
-               double* __restrict__ self_out, const double* __restrict__ skip) {
+               double* __restrict__ self_out, const double* __restrict__ skip, int hrow, double* __restrict__ Hk,
+               int ldh) {
   if (skip && *skip != 0.) return;
   __shared__ double red[kVecThreads / 32][kDotCols + 1];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -109,43 +183,17 @@ __global__ void __launch_bounds__(kVecThreads)
       }
     }
   }
-#pragma unroll
-  for (int c = 0; c < kDotCols; ++c) {
-    if (c < nc) {
-      const double t = warp_sum(acc[c]);
-      if (lane == 0) red[wid][c] = t;
-    }
+  {
+    const double t = warp_sum8<double>(
+        acc, [](double a, double b) { return a + b; },
+        [](double a, int o) { return __shfl_xor_sync(QDKGB_FULL_MASK, a, o); });
+    if ((lane & 3) == 0) red[wid][warp_sum8_col()] = t;
   }
   if (self) {
     const double t = warp_sum(accw);
     if (lane == 0) red[wid][kDotCols] = t;
   }
-  __syncthreads();
-  if (threadIdx.x < nc) {
-    double t = 0.;
-    for (int q = 0; q < kVecThreads / 32; ++q) t += red[q][threadIdx.x];
-    partial[(size_t)(j0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
-  }
-  if (self && threadIdx.x == kDotCols) {
-    double t = 0.;
-    for (int q = 0; q < kVecThreads / 32; ++q) t += red[q][kDotCols];
-    partial[(size_t)k * gridDim.x + blockIdx.x] = t;
-  }
-  if (!last_block_done(count, blockIdx.y, gridDim.x)) return;
-  if (wid < nc) {
-    const double* p = partial + (size_t)(j0 + wid) * gridDim.x;
-    double t = 0.;
-    for (int b = lane; b < (int)gridDim.x; b += 32) t += __ldcg(p + b);
-    t = warp_sum(t);
-    if (lane == 0) out[(size_t)(j0 + wid) * out_stride] = t;
-  }
-  if (self && wid == kVecThreads / 32 - 1) {
-    const double* p = partial + (size_t)k * gridDim.x;
-    double t = 0.;
-    for (int b = lane; b < (int)gridDim.x; b += 32) t += __ldcg(p + b);
-    t = warp_sum(t);
-    if (lane == 0) *self_out = t;
-  }
+  dot_finish(red, j0, nc, k, self, partial, count, out, out_stride, self_out, hrow, Hk, ldh);
 }
 // out[j * out_stride] = sum_b partial[j * nb + b], fixed order; one warp per j
 __global__ void k_reduce_partials(const double* __restrict__ partial, int nb, int k, double* out, int out_stride) {
@@ -163,13 +211,19 @@ __global__ void k_reduce_partials(const double* __restrict__ partial, int nb, in
 // reorthogonalisation test of a Gram-Schmidt pass (coef = V^T y for
 // orthonormal V, *w2 = |y|^2 before it): 1 when |y - V coef|^2 = *w2 - |coef|^2
 // keeps at least half of *w2 (a second pass is not needed), else 0.
-template <bool SUB>
+// NORM: *nrm_out = |y|^2 of the result, summed as k_multidot sums it (the same
+// rows per thread, trees and block order).
+template <bool SUB, bool NORM = false>
 __global__ void __launch_bounds__(kVecThreads)
     k_gemv_rows(const double* __restrict__ A, int64_t lda, int k, const double* __restrict__ coef, int coef_stride,
                 double* __restrict__ y, int64_t n, const double* __restrict__ skip = nullptr,
-                const double* __restrict__ w2 = nullptr, double* __restrict__ skip_out = nullptr) {
+                const double* __restrict__ w2 = nullptr, double* __restrict__ skip_out = nullptr,
+                double* __restrict__ partial = nullptr, unsigned* __restrict__ count = nullptr,
+                double* __restrict__ nrm_out = nullptr) {
   if (skip && *skip != 0.) return;
   __shared__ double c[kMaxSubspace + 2];
+  __shared__ double red[kVecThreads / 32][kDotCols + 1];
+  double yy = 0.;
   for (int j = threadIdx.x; j < k; j += blockDim.x) c[j] = coef[(size_t)j * coef_stride];
   __syncthreads();
   if (skip_out && blockIdx.x == 0 && threadIdx.x == 0) {
@@ -201,12 +255,20 @@ __global__ void __launch_bounds__(kVecThreads)
       if (has1) s1 = fma(A[i1 + (size_t)j * lda], c[j], s1);
     }
     if (SUB) {
-      y[i] -= s0;
-      if (has1) y[i1] -= s1;
-    } else {
-      y[i] = s0;
-      if (has1) y[i1] = s1;
+      s0 = y[i] - s0;
+      if (has1) s1 = y[i1] - s1;
     }
+    y[i] = s0;
+    if (has1) y[i1] = s1;
+    if (NORM) {
+      yy = fma(s0, s0, yy);
+      if (has1) yy = fma(s1, s1, yy);
+    }
+  }
+  if constexpr (NORM) {
+    const double t = warp_sum(yy);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][0] = t;
+    dot_finish(red, 0, 1, 1, false, partial, count, nrm_out, 1, nullptr, 0, nullptr, 0);
   }
 }
 // Y[:, o] = A[:, 0:k] Q[:, o] for o < nout <= kMaxOut (Q column-major, ld k):
@@ -272,7 +334,8 @@ __global__ void __launch_bounds__(kVecThreads)
     k_ritz_residual(const double* __restrict__ V, const double* __restrict__ AV, int64_t ld, int k,
                     const double* __restrict__ C0, const double* __restrict__ lam, double* __restrict__ X,
                     double* __restrict__ R, int64_t n, const double* __restrict__ D, double min_abs,
-                    double* __restrict__ partial, unsigned* __restrict__ count, double* __restrict__ out) {
+                    double* __restrict__ partial, unsigned* __restrict__ count, double* __restrict__ out,
+                    const double* __restrict__ flag) {
   __shared__ double c[kMaxSubspace + 2];
   __shared__ double red[kVecThreads / 32];
   for (int j = threadIdx.x; j < k; j += blockDim.x) c[j] = C0[j];
@@ -330,7 +393,13 @@ __global__ void __launch_bounds__(kVecThreads)
   for (int b = threadIdx.x; b < (int)gridDim.x; b += kVecThreads) u += __ldcg(partial + b);
   __syncthreads();
   u = block_sum_vec(u, red);
-  if (threadIdx.x == 0) *out = u;
+  if (threadIdx.x == 0) {
+    *out = u;
+    if (flag) {  // what the host reads with it
+      out[1] = l0;
+      out[2] = *flag;
+    }
+  }
 }
 // R = -R / (D - lam0) with |D - lam0| clamped to min_abs (davidson.hpp:352-361)
 __global__ void k_precondition(double* R, const double* __restrict__ D, const double* lam, int64_t n,
@@ -430,13 +499,6 @@ __global__ void __launch_bounds__(kFlipTile * 8) k_flip_project(double* x, int64
     }
   }
 }
-// Hk(i, c) = Hk(c, i) = v[c], c <= i
-__global__ void k_store_row(const double* v, int i, double* Hk, int ld) {
-  for (int c = threadIdx.x; c <= i; c += blockDim.x) {
-    Hk[i + (size_t)c * ld] = v[c];
-    Hk[c + (size_t)i * ld] = v[c];
-  }
-}
 
 // ---------------------------------------------------------------- double-float subspace
 // The mixed-precision solver keeps V, A V, the Ritz vector and the new
@@ -449,7 +511,8 @@ __global__ void k_store_row(const double* v, int i, double* Hk, int ld) {
 __global__ void __launch_bounds__(kVecThreads)
     k_df_multidot(const float2* __restrict__ A, int64_t lda, int k, const float2* __restrict__ w, int64_t n,
                   double* __restrict__ partial, unsigned* __restrict__ count, double* __restrict__ out, int out_stride,
-                  double* __restrict__ self_out, const double* __restrict__ skip) {
+                  double* __restrict__ self_out, const double* __restrict__ skip, int hrow, double* __restrict__ Hk,
+                  int ldh) {
   if (skip && *skip != 0.) return;
   __shared__ double red[kVecThreads / 32][kDotCols + 1];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -485,43 +548,31 @@ __global__ void __launch_bounds__(kVecThreads)
       }
     }
   }
+  {
+    // the exchange in double-float (48 bits, the FP32 pipe), the last steps in FP64
 #pragma unroll
-  for (int c = 0; c < kDotCols; ++c) {
-    if (c < nc) {
-      const double t = warp_sum(df::to_double(acc[c]));
-      if (lane == 0) red[wid][c] = t;
+    for (int c = 0; c < kDotCols; ++c) acc[c] = df::normalise(acc[c]);
+#pragma unroll
+    for (int h = 4; h >= 1; h >>= 1) {
+      const int o = 4 * h;
+      const bool up = lane & o;
+#pragma unroll
+      for (int q = 0; q < h; ++q) {
+        const float2 give = up ? acc[q] : acc[q + h], keep = up ? acc[q + h] : acc[q];
+        acc[q] = df::add(keep, make_float2(__shfl_xor_sync(QDKGB_FULL_MASK, give.x, o),
+                                           __shfl_xor_sync(QDKGB_FULL_MASK, give.y, o)));
+      }
     }
+    double t = df::to_double(acc[0]);
+    t += __shfl_xor_sync(QDKGB_FULL_MASK, t, 2);
+    t += __shfl_xor_sync(QDKGB_FULL_MASK, t, 1);
+    if ((lane & 3) == 0) red[wid][warp_sum8_col()] = t;
   }
   if (self) {
     const double t = warp_sum(df::to_double(accw));
     if (lane == 0) red[wid][kDotCols] = t;
   }
-  __syncthreads();
-  if (threadIdx.x < nc) {
-    double t = 0.;
-    for (int q = 0; q < kVecThreads / 32; ++q) t += red[q][threadIdx.x];
-    partial[(size_t)(j0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
-  }
-  if (self && threadIdx.x == kDotCols) {
-    double t = 0.;
-    for (int q = 0; q < kVecThreads / 32; ++q) t += red[q][kDotCols];
-    partial[(size_t)k * gridDim.x + blockIdx.x] = t;
-  }
-  if (!last_block_done(count, blockIdx.y, gridDim.x)) return;
-  if (wid < nc) {
-    const double* p = partial + (size_t)(j0 + wid) * gridDim.x;
-    double t = 0.;
-    for (int b = lane; b < (int)gridDim.x; b += 32) t += __ldcg(p + b);
-    t = warp_sum(t);
-    if (lane == 0) out[(size_t)(j0 + wid) * out_stride] = t;
-  }
-  if (self && wid == kVecThreads / 32 - 1) {
-    const double* p = partial + (size_t)k * gridDim.x;
-    double t = 0.;
-    for (int b = lane; b < (int)gridDim.x; b += 32) t += __ldcg(p + b);
-    t = warp_sum(t);
-    if (lane == 0) *self_out = t;
-  }
+  dot_finish(red, j0, nc, k, self, partial, count, out, out_stride, self_out, hrow, Hk, ldh);
 }
 // y -= A[:, 0:k] coef (k_gemv_rows<true> in double-float; the same skip and
 // selective-reorthogonalisation outputs).  nrm_out, when given, receives
@@ -638,7 +689,8 @@ __global__ void __launch_bounds__(kVecThreads)
     k_df_ritz_residual(const float2* __restrict__ V, const float2* __restrict__ AV, int64_t ld, int k,
                        const double* __restrict__ C0, const double* __restrict__ lam, float2* __restrict__ X,
                        float2* __restrict__ R, int64_t n, const float2* __restrict__ Dd, double min_abs,
-                       double* __restrict__ partial, unsigned* __restrict__ count, double* __restrict__ out) {
+                       double* __restrict__ partial, unsigned* __restrict__ count, double* __restrict__ out,
+                       const double* __restrict__ flag) {
   __shared__ float2 c[kMaxSubspace + 2];
   __shared__ double red[kVecThreads / 32];
   for (int j = threadIdx.x; j < k; j += blockDim.x) c[j] = df::split(C0[j]);
@@ -705,7 +757,11 @@ __global__ void __launch_bounds__(kVecThreads)
   for (int b = threadIdx.x; b < (int)gridDim.x; b += kVecThreads) u += __ldcg(partial + b);
   __syncthreads();
   u = block_sum_vec(u, red);
-  if (threadIdx.x == 0) *out = u;
+  if (threadIdx.x == 0) {
+    *out = u;
+    out[1] = lam[0];
+    out[2] = *flag;
+  }
 }
 __global__ void k_df_from_f64(const double* __restrict__ x, float2* __restrict__ y, int64_t n) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -799,7 +855,7 @@ void lowest_eig_batch(cudaStream_t st, int B, const int* kdev, int kadd, int kma
 namespace {
 
 // slots in the small scratch array
-constexpr int kSlotRes = kMaxSubspace + 4;   // residual norm^2 (device reduce target)
+constexpr int kSlotRes = kMaxSubspace + 4;   // residual norm^2 (device reduce target), Ritz value, Gram-Schmidt flag
 constexpr int kSlotNrm = kMaxSubspace + 8;   // Gram-Schmidt norm^2
 constexpr int kSlotE = kMaxSubspace + 12;    // full-precision Rayleigh quotient
 constexpr int kSlotFlag = kMaxSubspace + 16; // Gram-Schmidt degeneracy flag
@@ -828,11 +884,11 @@ struct Dav {
   // grid.y, the row split on grid.x shrunk as column blocks are added (down to
   // one block per SM) so the grid stays near one resident wave
   void multidot(const double* A, int k, const double* w, double* out, int stride, double* self_out = nullptr,
-                const double* skip = nullptr) {
+                const double* skip = nullptr, int hrow = -1) {
     const int chunks = (k + kDotCols - 1) / kDotCols;
     const int bx = std::max(1, std::min(nb, std::max(sm_count, nb / chunks)));
     k_multidot<<<dim3(bx, chunks), kVecThreads, 0, st>>>(A, n, k, w, n, partial, counts(), out, stride, self_out,
-                                                         skip);
+                                                         skip, hrow, hrow >= 0 ? Hk : nullptr, (int)(maxm + 1));
     QDKGB_CHECK_LAUNCH();
   }
   void norm2(const double* w, double* out) { multidot(w, 1, w, out, 1); }
@@ -841,6 +897,20 @@ struct Dav {
     QDKGB_CUDA(cudaMemcpyAsync(c->pinned, a, sizeof(double), cudaMemcpyDeviceToHost, st));
     QDKGB_CUDA(cudaStreamSynchronize(st));
     va = c->pinned[0];
+  }
+  // What a Ritz step left for the host (residual norm^2, lowest Ritz value, the
+  // pending Gram-Schmidt flag): the copy goes out with ask(), answer() waits for
+  // it alone, so that work enqueued in between runs on.
+  cudaEvent_t asked = nullptr;
+  void ask() {
+    QDKGB_CUDA(cudaMemcpyAsync(c->pinned, small + kSlotRes, 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
+    QDKGB_CUDA(cudaEventRecord(asked, st));
+  }
+  void answer(double& r2, double& lam, bool& flag) {
+    QDKGB_CUDA(cudaEventSynchronize(asked));
+    r2 = c->pinned[0];
+    lam = c->pinned[1];
+    flag = c->pinned[2] != 0.;
   }
   // residual norm^2, lowest Ritz value and the pending Gram-Schmidt flag in one sync
   void fetch3(const double* a, const double* b, double& va, double& vb, bool& flag) {
@@ -854,34 +924,26 @@ struct Dav {
   }
   void clear_flag() { QDKGB_CUDA(cudaMemsetAsync(small + kSlotFlag, 0, sizeof(double), st)); }
 
-  // Two CGS passes against V[:, 0:K].  selective: the second pass only when
-  // the first removed more than half of |w|^2 (the Daniel-Gragg-Kaufman-
-  // Stewart test, decided on the device; the mixed path's choice - the
-  // reference always makes two passes).
-  void orth_passes(int K, double* w, bool selective = false) {
-    if (K <= 0) return;
-    if (!selective) {
-      for (int pass = 0; pass < 2; ++pass) {
-        multidot(V, K, w, small, 1);
-        k_gemv_rows<true><<<nb, kVecThreads, 0, st>>>(V, n, K, small, 1, w, n);
-        QDKGB_CHECK_LAUNCH();
-      }
+  // Two CGS passes against V[:, 0:K] (the reference always makes two).
+  // |w|^2 of the result goes to small[kSlotNrm].
+  void orth_passes(int K, double* w) {
+    if (K <= 0) {
+      norm2(w, small + kSlotNrm);
       return;
     }
-    multidot(V, K, w, small, 1, small + kSlotW2);
-    k_gemv_rows<true><<<nb, kVecThreads, 0, st>>>(V, n, K, small, 1, w, n, nullptr, small + kSlotW2,
-                                                  small + kSlotSkip);
+    multidot(V, K, w, small, 1);
+    k_gemv_rows<true><<<nb, kVecThreads, 0, st>>>(V, n, K, small, 1, w, n);
     QDKGB_CHECK_LAUNCH();
-    multidot(V, K, w, small, 1, nullptr, small + kSlotSkip);
-    k_gemv_rows<true><<<nb, kVecThreads, 0, st>>>(V, n, K, small, 1, w, n, small + kSlotSkip);
+    multidot(V, K, w, small, 1);
+    k_gemv_rows<true, true><<<nb, kVecThreads, 0, st>>>(V, n, K, small, 1, w, n, nullptr, nullptr, nullptr, partial,
+                                                        counts(), small + kSlotNrm);
     QDKGB_CHECK_LAUNCH();
   }
   // gram_schmidt (davidson.hpp:185-238): two CGS passes against V[:, 0:K],
   // normalise; a degenerate result raises the device flag (checked at the
   // next host sync, then repaired by fallback()).
-  void gram_schmidt(int K, double* w, double min_norm = 1e-12, bool selective = false) {
-    orth_passes(K, w, selective);
-    norm2(w, small + kSlotNrm);
+  void gram_schmidt(int K, double* w, double min_norm = 1e-12) {
+    orth_passes(K, w);
     k_normalize<<<nb, 256, 0, st>>>(w, n, small + kSlotNrm, min_norm, small + kSlotFlag);
     QDKGB_CHECK_LAUNCH();
   }
@@ -892,7 +954,6 @@ struct Dav {
       const double one = 1.0;
       QDKGB_CUDA(cudaMemcpyAsync(w + idx, &one, sizeof(double), cudaMemcpyHostToDevice, st));
       orth_passes(K, w);
-      norm2(w, small + kSlotNrm);
       double nv;
       fetch(small + kSlotNrm, nv);
       if (std::sqrt(nv) > min_norm) {
@@ -927,9 +988,7 @@ struct Dav {
   // new row i of the projected matrix, Hk(i, c) = V_i . AV_c for c <= i,
   // mirrored (syev reads the lower triangle, rayleigh_ritz.hpp:70-77)
   void projected_row(int i) {
-    multidot(AV, i + 1, col(V, i), small, 1);
-    k_store_row<<<1, 256, 0, st>>>(small, i, Hk, (int)(maxm + 1));
-    QDKGB_CHECK_LAUNCH();
+    multidot(AV, i + 1, col(V, i), nullptr, 1, nullptr, nullptr, i);
   }
 
   // X = V C0, R = AV C0 - lam0 X with |R|^2 into small[kSlotRes]; R is
@@ -937,7 +996,7 @@ struct Dav {
   // orthogonalisation)
   void ritz_residual(int k, double* R, double min_abs) {
     k_ritz_residual<<<nb, kVecThreads, 0, st>>>(V, AV, n, k, evec, eval, X, R, n, D, min_abs, partial, counts(),
-                                                small + kSlotRes);
+                                                small + kSlotRes, small + kSlotFlag);
     QDKGB_CHECK_LAUNCH();
   }
   // ---- the double-float subspace of the mixed-precision solver
@@ -948,7 +1007,7 @@ struct Dav {
   // (its sixteen loads in flight per thread take more registers than four
   // blocks per SM allow)
   void df_multidot(const float2* A, int k, const float2* w, double* out, int stride, double* self_out = nullptr,
-                   const double* skip = nullptr) {
+                   const double* skip = nullptr, int hrow = -1) {
     static const int per_sm = [] {
       int b = 0;
       QDKGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_df_multidot, kVecThreads, 0));
@@ -958,7 +1017,7 @@ struct Dav {
     const int chunks = (k + kDotCols - 1) / kDotCols;
     const int bx = std::max(1, std::min(nbd, std::max(sm_count, nbd / chunks)));
     k_df_multidot<<<dim3(bx, chunks), kVecThreads, 0, st>>>(A, n, k, w, n, partial, counts(), out, stride, self_out,
-                                                            skip);
+                                                            skip, hrow, hrow >= 0 ? Hk : nullptr, (int)(maxm + 1));
     QDKGB_CHECK_LAUNCH();
   }
   // the two CGS passes of df_gram_schmidt; every update that runs leaves
@@ -1013,13 +1072,11 @@ struct Dav {
     throw Error(QDKGB_ERR_INVALID, "gram_schmidt: Unable to find orthogonal vector");
   }
   void df_projected_row(int i) {
-    df_multidot(AVf, i + 1, colf(Vf, i), small, 1);
-    k_store_row<<<1, 256, 0, st>>>(small, i, Hk, (int)(maxm + 1));
-    QDKGB_CHECK_LAUNCH();
+    df_multidot(AVf, i + 1, colf(Vf, i), nullptr, 1, nullptr, nullptr, i);
   }
   void df_ritz_residual(int k, float2* Xr, float2* R, const float2* Dd, double min_abs) {
     k_df_ritz_residual<<<nb, kVecThreads, 0, st>>>(Vf, AVf, n, k, evec, eval, Xr, R, n, Dd, min_abs, partial, counts(),
-                                                   small + kSlotRes);
+                                                   small + kSlotRes, small + kSlotFlag);
     QDKGB_CHECK_LAUNCH();
   }
   void df_from_f64(const double* x, float2* y) {
@@ -1036,7 +1093,7 @@ struct Dav {
   // small[kSlotRoots + r]
   void ritz_residual_root(int k, int r, double* Xr, double* Rr, double min_abs) {
     k_ritz_residual<<<nb, kVecThreads, 0, st>>>(V, AV, n, k, evec + (size_t)r * k, eval + r, Xr, Rr, n, D, min_abs,
-                                                partial, counts(), small + kSlotRoots + r);
+                                                partial, counts(), small + kSlotRoots + r, nullptr);
     QDKGB_CHECK_LAUNCH();
   }
 };
@@ -1292,6 +1349,20 @@ void davidson(Context* c, const qdkgb_davidson_settings* s, double* E, double* C
 
   double lam0 = 0., res = 0.;
   bool converged = false;
+  struct Asked {
+    cudaEvent_t e = nullptr;
+    ~Asked() {
+      if (e) cudaEventDestroy(e);
+    }
+  } asked;
+  QDKGB_CUDA(cudaEventCreateWithFlags(&asked.e, cudaEventDisableTiming));
+  d.asked = asked.e;
+  // The next direction and its sigma are enqueued before the host has read the
+  // residual, so that the GPU does not wait for the host's answer (20-30 us an
+  // iteration, as long as a small space's whole Gram-Schmidt), unless the last
+  // residual was within kAhead of the tolerance: a step that turns out to be
+  // the last leaves at most work that nobody needs.
+  constexpr double kAhead = 8.;
 
   if (!mixed) {
     // ---------------- plain FP64 Davidson: the reference's algorithm
@@ -1301,17 +1372,31 @@ void davidson(Context* c, const qdkgb_davidson_settings* s, double* E, double* C
     d.gram_schmidt(1, d.col(d.V, 1));
     d.projected_row(0);
     int64_t iter = 1;
+    bool ahead = false;  // V[:, i], its sigma and its projected row are there already
+    double last = 1e300;
     for (int64_t i = 1; i < max_m; ++i, ++iter) {
       const int k = (int)i + 1;
-      sigma_full(d.col(d.V, i), d.col(d.AV, i));
-      d.projected_row((int)i);
+      if (!ahead) {
+        sigma_full(d.col(d.V, i), d.col(d.AV, i));
+        d.projected_row((int)i);
+      }
       d.lowest(k);
       double* R = d.col(d.V, i + 1);
       d.ritz_residual(k, R, s->min_abs_denominator);
+      d.ask();
+      ahead = last > kAhead * s->res_tol && i + 1 < max_m;
+      if (ahead) {
+        d.gram_schmidt(k, R);
+        sigma_full(R, d.col(d.AV, i + 1));
+        d.projected_row((int)i + 1);
+      }
       double r2 = 0.;
       bool degenerate = false;
-      d.fetch3(d.small + kSlotRes, d.eval, r2, lam0, degenerate);
+      d.answer(r2, lam0, degenerate);
+      last = std::sqrt(r2);
       if (degenerate) {
+        if (ahead) loc.spmv_fp64--;
+        ahead = false;
         // V[:, i] was not normalisable: repair it and redo this iteration
         d.fallback((int)i, d.col(d.V, i));
         d.forget_warm();
@@ -1323,9 +1408,10 @@ void davidson(Context* c, const qdkgb_davidson_settings* s, double* E, double* C
       loc.iterations = iter;
       if (res < s->res_tol) {
         converged = true;
+        if (ahead) loc.spmv_fp64--;
         break;
       }
-      d.gram_schmidt(k, R);
+      if (!ahead) d.gram_schmidt(k, R);
     }
   } else {
     // ---------------- mixed: FP32 sigma for new directions, full-precision refresh
@@ -1407,22 +1493,38 @@ void davidson(Context* c, const qdkgb_davidson_settings* s, double* E, double* C
     double best = 1e300;
     int since_best = 0;
     bool have_x64 = false;  // d.X holds the FP64 copy of the current Ritz vector
-    while (iter < 4 * max_m) {
+    // column k of A V and its projected row from the direction in V[:, k] / xf
+    auto extend = [&](int kc) {
       spmv_fp32(c, xf, yf);
       loc.spmv_fp32++;
-      k_df_from_f32<<<d.nb, 256, 0, c->stream>>>(yf, d.colf(d.AVf, k), N);
+      k_df_from_f32<<<d.nb, 256, 0, c->stream>>>(yf, d.colf(d.AVf, kc), N);
       QDKGB_CHECK_LAUNCH();
-      d.df_projected_row(k);
+      d.df_projected_row(kc);
+    };
+    bool ahead = false;
+    double last = 1e300;
+    while (iter < 4 * max_m) {
+      if (!ahead) extend(k);
       ++k;
       ++iter;
       d.lowest(k);
       float2* R = (k <= max_m - 1) ? d.colf(d.Vf, k) : Rtf;
       d.df_ritz_residual(k, Xf, R, Df, s->min_abs_denominator);
       have_x64 = false;
+      d.ask();
+      ahead = last > kAhead * std::max(0.5 * s->res_tol, drop * last_true) && since_best < 4 && k < max_m - 2;
+      if (ahead) {
+        project(R);
+        d.df_gram_schmidt(k, R, 1e-12, true);
+        extend(k);
+      }
       double r2 = 0.;
       bool degenerate = false;
-      d.fetch3(d.small + kSlotRes, d.eval, r2, lam0, degenerate);
+      d.answer(r2, lam0, degenerate);
+      last = std::sqrt(r2);
       if (degenerate) {
+        if (ahead) loc.spmv_fp32--;
+        ahead = false;
         --k;
         --iter;
         d.df_fallback(k, d.colf(d.Vf, k));
@@ -1440,10 +1542,18 @@ void davidson(Context* c, const qdkgb_davidson_settings* s, double* E, double* C
       const bool refresh =
           est < 0.5 * s->res_tol || est < drop * last_true || since_best >= 6 || k >= max_m - 1;
       if (!refresh) {
-        project(R);
-        d.df_gram_schmidt(k, R, 1e-12, true);
+        if (!ahead) {
+          project(R);
+          d.df_gram_schmidt(k, R, 1e-12, true);
+        }
         continue;
       }
+      if (ahead) {  // the direction beyond the refreshed vector is not used
+        loc.spmv_fp32--;
+        d.clear_flag();
+      }
+      ahead = false;
+      last = 1e300;
       // full-precision sigma, Rayleigh quotient and residual of X (unit norm)
       d.df_to_f64(Xf, d.X);
       have_x64 = true;
