@@ -296,6 +296,7 @@ int qdkgb_destroy(qdkgb_context* c) {
                           &c->dav.evec, &c->dav.eval, &c->dav.scratch, &c->dav.partial, &c->dav.small, &c->dav.eig})
     dev_free(c, *b);
   free_direct(c);
+  free_rdm(c);
   free_struct(c);
   if (c->pinned) cudaFreeHost(c->pinned);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);

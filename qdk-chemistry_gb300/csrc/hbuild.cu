@@ -256,6 +256,7 @@ void build_det_space(Context* c, int64_t nd, const uint64_t* alpha, const uint64
   c->fci_shape[0] = c->fci_shape[1] = c->fci_shape[2] = -1;
   c->H.valid = false;
   free_direct(c);
+  free_rdm(c);
   free_struct(c);
   c->op_direct = false;
   c->fp32_direct = c->fp64_direct = false;

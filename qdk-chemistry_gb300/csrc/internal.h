@@ -56,6 +56,7 @@ struct Context;
 struct Integrals;
 struct DirectSigma;
 struct FciStruct;
+struct RdmPlan;
 
 void count_launch();
 // cudaFuncAttributeMaxDynamicSharedMemorySize of a kernel on the current
@@ -144,6 +145,7 @@ struct Context {
   Hcsr H;
   DavidsonWork dav;
   DirectSigma* direct = nullptr;  // recompute-on-the-fly operator (complete spaces)
+  RdmPlan* rdm = nullptr;         // string lists and workspaces of a complete space's RDMs
   FciStruct* fci = nullptr;       // row-shape tables of a complete space (structured kernels)
   bool op_direct = false;         // Davidson / spmv use the direct sigma instead of the CSR
   bool fp32_direct = false;       // complete space, mixed form: FP32 sigma by the direct contraction,
@@ -301,6 +303,7 @@ void davidson(Context* c, const qdkgb_davidson_settings* s, double* E, double* C
               bool steady = false);
 
 // rdm.cu
+void free_rdm(Context* c);
 void rdms_spin_dep(Context* c, const double* C, double* aa, double* bb, double* aaaa, double* bbbb, double* aabb);
 void orbital_entropies(Context* c, const double* C, double* s1, double* s2, double* mi);
 

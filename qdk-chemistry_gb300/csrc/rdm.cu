@@ -18,6 +18,8 @@
 #include <limits>
 #include <vector>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "internal.h"
 #include "rowwalk.cuh"
@@ -263,63 +265,113 @@ __device__ __forceinline__ double cas_acc(double acc, double a, double b, bool n
   return fabs(p) > 1e-16 ? acc + flip_if(p, neg) : acc;
 }
 
+// Two alpha transitions at a time: their rows of C interleaved in shared
+// memory (one 16-byte read serves both), each list entry read and decoded once
+// for the two.  The lists are transposed ([entry][item], padded with the entry
+// (nb, nb) whose row elements are zero), so a warp reads 128 contiguous bytes;
+// a thread walking its own list would touch a sector per lane, and those
+// reads would share the pace with the FP64 pipe (two lanes a clock, the bound
+// now; CASCI(12,12): 2.15 ms before, 1.63 ms).  TWO = false: spaces whose
+// four rows do not fit in shared memory, one transition at a time.
+// DIAG: the string-diagonal alpha transitions.  Their t_ij(gI) is the same for
+// every orbital that gI occupies, so it is formed once per string (two strings
+// per CTA; partial[gI][item]) and k_rdm_cas_ab_reduce adds the strings of each
+// orbital: n_alpha times fewer of these transitions (CASCI(12,12): 17,556
+// transitions in all instead of 22,176).
+template <bool TWO, bool DIAG>
 __global__ void __launch_bounds__(kCasThreads)
     k_rdm_cas_ab(int64_t nb, const double* __restrict__ C, const uint32_t* __restrict__ atr,
-                 const int4* __restrict__ chunks, const CasItem* __restrict__ items, int nitems,
-                 const uint32_t* __restrict__ blist, double* __restrict__ partial) {
-  extern __shared__ double rows[];  // rowI | rowJ
-  double* rowI = rows;
-  double* rowJ = rows + nb;
-  const int4 ch = chunks[blockIdx.x];  // (alpha class, first transition, count, unused)
+                 const int4* __restrict__ chunks, int nitems, int istride, int len, const uint32_t* __restrict__ blist,
+                 double* __restrict__ partial) {
+  extern __shared__ __align__(16) unsigned char rdm_smem[];
+  using Row = typename std::conditional<TWO, double2, double>::type;
+  Row* rowI = (Row*)rdm_smem;  // [nb + 1], the last one zero
+  Row* rowJ = rowI + nb + 1;
+  auto first = [](const Row& r) {
+    if constexpr (TWO) return r.x;
+    else return r;
+  };
+  // (alpha class, first transition, count, string count)
+  const int4 ch = DIAG ? make_int4(0, 0, TWO ? 2 : 1, chunks[0].w) : chunks[blockIdx.x];
+  const int g0 = (TWO ? 2 : 1) * blockIdx.x;
   const int it = threadIdx.x;
-  CasItem item = {0, 0, 0};
-  if (it < nitems) item = items[it];
-  const uint32_t* lst = blist + item.begin;
+  const uint32_t* lst = blist + min(it, istride - 1);
+  const bool mine = it < nitems;
   double acc = 0.;
-  for (int t = 0; t < ch.z; ++t) {
-    const uint32_t w = __ldg(atr + ch.y + t);
-    const int64_t gI = w & 0x7fff, gJ = (w >> 15) & 0x7fff;
-    const bool na = (w >> 31) != 0;
+  if (threadIdx.x == 0) rowI[nb] = rowJ[nb] = Row{};
+  for (int t = 0; t < ch.z; t += TWO ? 2 : 1) {
+    const bool two = TWO && (DIAG ? g0 + 1 < ch.w : t + 1 < ch.z);
+    const uint32_t w0 = DIAG ? (uint32_t)(g0 | (g0 << 15)) : __ldg(atr + ch.y + t);
+    const uint32_t w1 = !two ? w0 : DIAG ? (uint32_t)((g0 + 1) | ((g0 + 1) << 15)) : __ldg(atr + ch.y + t + 1);
+    const double *i0 = C + (int64_t)(w0 & 0x7fff) * nb, *j0 = C + (int64_t)((w0 >> 15) & 0x7fff) * nb;
+    const double *i1 = C + (int64_t)(w1 & 0x7fff) * nb, *j1 = C + (int64_t)((w1 >> 15) & 0x7fff) * nb;
     __syncthreads();
     for (int64_t b = threadIdx.x; b < nb; b += blockDim.x) {
-      rowI[b] = C[gI * nb + b];
-      rowJ[b] = C[gJ * nb + b];
+      if constexpr (TWO) {
+        rowI[b] = make_double2(i0[b], two ? i1[b] : 0.);
+        rowJ[b] = make_double2(j0[b], two ? j1[b] : 0.);
+      } else {
+        rowI[b] = i0[b];
+        rowJ[b] = j0[b];
+      }
     }
     __syncthreads();
-    double s0 = 0., s1 = 0., s2 = 0., s3 = 0.;
-    int e = 0;
-    for (; e + 4 <= item.len; e += 4) {
-      const uint32_t x0 = __ldg(lst + e), x1 = __ldg(lst + e + 1), x2 = __ldg(lst + e + 2), x3 = __ldg(lst + e + 3);
-      s0 = cas_acc(s0, rowI[x0 & 0x7fff], rowJ[(x0 >> 15) & 0x7fff], (x0 >> 31) != 0);
-      s1 = cas_acc(s1, rowI[x1 & 0x7fff], rowJ[(x1 >> 15) & 0x7fff], (x1 >> 31) != 0);
-      s2 = cas_acc(s2, rowI[x2 & 0x7fff], rowJ[(x2 >> 15) & 0x7fff], (x2 >> 31) != 0);
-      s3 = cas_acc(s3, rowI[x3 & 0x7fff], rowJ[(x3 >> 15) & 0x7fff], (x3 >> 31) != 0);
+    if (mine) {
+      double s0 = 0., s1 = 0., u0 = 0., u1 = 0.;
+      int e = 0;
+#pragma unroll 2
+      for (; e + 2 <= len; e += 2) {
+        const uint32_t x = __ldg(lst + (int64_t)e * istride), y = __ldg(lst + (int64_t)(e + 1) * istride);
+        const Row a = rowI[x & 0x7fff], b = rowJ[(x >> 15) & 0x7fff];
+        const Row c = rowI[y & 0x7fff], d = rowJ[(y >> 15) & 0x7fff];
+        s0 = cas_acc(s0, first(a), first(b), (x >> 31) != 0);
+        u0 = cas_acc(u0, first(c), first(d), (y >> 31) != 0);
+        if constexpr (TWO) {
+          s1 = cas_acc(s1, a.y, b.y, (x >> 31) != 0);
+          u1 = cas_acc(u1, c.y, d.y, (y >> 31) != 0);
+        }
+      }
+      if (e < len) {
+        const uint32_t x = __ldg(lst + (int64_t)e * istride);
+        const Row a = rowI[x & 0x7fff], b = rowJ[(x >> 15) & 0x7fff];
+        s0 = cas_acc(s0, first(a), first(b), (x >> 31) != 0);
+        if constexpr (TWO) s1 = cas_acc(s1, a.y, b.y, (x >> 31) != 0);
+      }
+      if (DIAG) {
+        partial[(int64_t)g0 * nitems + it] = s0 + u0;
+        if (two) partial[(int64_t)(g0 + 1) * nitems + it] = s1 + u1;
+        return;
+      }
+      acc += flip_if(s0 + u0, (w0 >> 31) != 0);
+      if (TWO) acc += flip_if(s1 + u1, (w1 >> 31) != 0);
     }
-    for (; e < item.len; ++e) {
-      const uint32_t x0 = __ldg(lst + e);
-      s0 = cas_acc(s0, rowI[x0 & 0x7fff], rowJ[(x0 >> 15) & 0x7fff], (x0 >> 31) != 0);
-    }
-    acc += flip_if((s0 + s1) + (s2 + s3), na);
   }
-  if (it < nitems) partial[(int64_t)blockIdx.x * nitems + it] = acc;
+  if (mine && !DIAG) partial[(int64_t)blockIdx.x * nitems + it] = acc;
 }
 
 // G[i, j, k, l] (and G[j, i, l, k] for k > l) = 1/2 sum over the class's
-// chunks and the beta class's items, in a fixed order.  One thread per
-// (alpha class, beta class).
+// chunks (k = l: the strings of its transitions, acls_chunks their range in
+// atr) and the beta class's items, in a fixed order.  One warp per (alpha
+// class, beta class).
 __global__ void k_rdm_cas_ab_reduce(int n, int nacls, const int2* __restrict__ acls, const int2* __restrict__ acls_chunks,
                                     const int2* __restrict__ bcls_items, int nitems,
-                                    const double* __restrict__ partial, double* __restrict__ G) {
+                                    const double* __restrict__ partial, const uint32_t* __restrict__ atr,
+                                    const double* __restrict__ diag, double* __restrict__ G) {
   const int n2 = n * n;
-  const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (tid >= (int64_t)nacls * n2) return;
-  const int ac = (int)(tid / n2), bc = (int)(tid % n2);
+  const int64_t id = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (id >= (int64_t)nacls * n2) return;
+  const int ac = (int)(id / n2), bc = (int)(id % n2);
   const int2 kl = acls[ac];
   const int2 chr = acls_chunks[ac];
   const int2 itr = bcls_items[bc];
   double v = 0.;
-  for (int q = chr.x; q < chr.y; ++q)
-    for (int m = itr.x; m < itr.y; ++m) v += partial[(int64_t)q * nitems + m];
+  for (int q = chr.x + lane; q < chr.y; q += 32) {
+    const double* row = kl.x == kl.y ? diag + (int64_t)(__ldg(atr + q) & 0x7fff) * nitems : partial + (int64_t)q * nitems;
+    for (int m = itr.x; m < itr.y; ++m) v += row[m];
+  }
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane) return;
   v *= 0.5;
   const int i = bc % n, j = bc / n, k = kl.x, l = kl.y;
   G[i + (size_t)n * (j + (size_t)n * (k + (size_t)n * l))] = v;
@@ -327,20 +379,37 @@ __global__ void k_rdm_cas_ab_reduce(int n, int nacls, const int2* __restrict__ a
 }
 
 // S[p] = sum_b X[r1, b] X[r2, b] over the pair list (rows of X with ld cols),
-// each product kept when |product| > 1e-16.  One warp per pair.
-__global__ void k_pair_overlap(int64_t npairs, const int2* __restrict__ pairs, const double* __restrict__ X,
-                               int64_t cols, double* __restrict__ S) {
-  const int lane = threadIdx.x & 31;
-  for (int64_t p = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; p < npairs;
-       p += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-    const int2 pr = pairs[p];
-    const double* x = X + pr.x * cols;
-    const double* y = X + pr.y * cols;
-    double s = 0.;
-    for (int64_t b = lane; b < cols; b += 32) {
-      const double v = __ldg(x + b) * __ldg(y + b);
-      if (fabs(v) > 1e-16) s += v;
+// each product kept when |product| > 1e-16 (cas_acc: one FP64 operation where
+// the exponents decide, where the product, its test and the sum were three).
+// One CTA per string r1, whose row stays in shared memory for all of its
+// pairs (begin[r1] ..); a warp per pair.  CASCI(12,12): 0.68 -> 0.30 ms a spin
+// (0.19 ms at two lanes a clock).
+__global__ void __launch_bounds__(256)
+    k_pair_overlap(const int* __restrict__ begin, const int2* __restrict__ pairs, const double* __restrict__ X,
+                   int64_t cols, int staged, double* __restrict__ S) {
+  extern __shared__ __align__(16) unsigned char rdm_smem[];
+  double* row = (double*)rdm_smem;
+  const int lane = threadIdx.x & 31, r = blockIdx.x;
+  const double* x = X + r * cols;
+  if (staged) {
+    for (int64_t b = threadIdx.x; b < cols; b += 256) row[b] = x[b];
+    __syncthreads();
+    x = row;
+  }
+  const int p1 = __ldg(begin + r + 1);
+  for (int p = __ldg(begin + r) + (threadIdx.x >> 5); p < p1; p += 8) {
+    const double* y = X + (int64_t)pairs[p].y * cols;
+    double s = 0., u = 0.;
+    int64_t b = lane;
+    for (; b + 96 < cols; b += 128) {
+      const double y0 = __ldg(y + b), y1 = __ldg(y + b + 32), y2 = __ldg(y + b + 64), y3 = __ldg(y + b + 96);
+      s = cas_acc(s, x[b], y0, false);
+      u = cas_acc(u, x[b + 32], y1, false);
+      s = cas_acc(s, x[b + 64], y2, false);
+      u = cas_acc(u, x[b + 96], y3, false);
     }
+    for (; b < cols; b += 32) s = cas_acc(s, x[b], __ldg(y + b), false);
+    s += u;
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) S[p] = s;
   }
@@ -392,64 +461,118 @@ static void cas_string_maps(const std::vector<uint64_t>& strs, std::vector<int32
   for (size_t i = 0; i < strs.size(); ++i) rank_of[strs[i]] = (int32_t)i;
 }
 
-// Returns false (nothing accumulated) when the space has more beta classes
-// than the kernel's CTA holds; the pair walk serves it then.
-static bool rdms_cas(Context* c, const double* dC, double* aa, double* bb, double* aaaa, double* bbbb, double* aabb) {
+}  // namespace qdkgb
+
+namespace qdkgb {
+
+// What the RDMs of a complete space need besides the vector: the transition
+// and pair lists of its strings (made once per determinant list and orbital
+// count), and the workspaces, which stay while they are small (kRdmKeep) and
+// the context's memory is not capped.
+struct RdmPlan {
+  int n = 0;
+  bool ab = false;         // the opposite-spin sweep serves this space
+  int nitems = 0, istride = 0, len = 0, nacls = 0, nchunks = 0;
+  DeviceBuffer bl, at, ch, ac, acc, bi;
+  struct Spin {
+    int64_t np = 0;
+    DeviceBuffer pairs, begin, str;
+  } spin[2];
+  DeviceBuffer C, Ct, G, part, S, t4, t2;
+};
+constexpr size_t kRdmKeep = (size_t)256 << 20;
+
+void free_rdm(Context* c) {
+  if (!c->rdm) return;
+  RdmPlan* p = c->rdm;
+  for (DeviceBuffer* b : {&p->bl, &p->at, &p->ch, &p->ac, &p->acc, &p->bi, &p->C, &p->Ct, &p->G, &p->part, &p->S, &p->t4,
+                          &p->t2, &p->spin[0].pairs, &p->spin[0].begin, &p->spin[0].str, &p->spin[1].pairs,
+                          &p->spin[1].begin, &p->spin[1].str})
+    dev_free(c, *b);
+  delete p;
+  c->rdm = nullptr;
+}
+static void trim_rdm(Context* c) {
+  RdmPlan* p = c->rdm;
+  size_t held = 0;
+  for (DeviceBuffer* b : {&p->C, &p->Ct, &p->G, &p->part, &p->S, &p->t4, &p->t2}) held += b->bytes;
+  if (c->dev_limit > 0)
+    free_rdm(c);
+  else if (held > kRdmKeep)
+    for (DeviceBuffer* b : {&p->C, &p->Ct, &p->G, &p->part, &p->S, &p->t4, &p->t2}) dev_free(c, *b);
+}
+
+// The plan of the context's space; ab false when the space has more beta
+// classes than the sweep's CTA holds (the pair walk serves it then).
+static RdmPlan* rdm_plan(Context* c) {
+  if (c->rdm && c->rdm->n == c->norb) return c->rdm;
+  free_rdm(c);
   const DetSpace& S = c->dets;
   const int n = c->norb;
-  const int64_t na = S.ngroups, nb = S.nbeta, N = na * nb;
-  const size_t n2 = (size_t)n * n, n4 = n2 * n2;
+  const int64_t na = S.ngroups, nb = S.nbeta;
+  const size_t n2 = (size_t)n * n;
+  RdmPlan* P = c->rdm = new RdmPlan();
+  P->n = n;
   std::vector<int32_t> ra, rb;
   cas_string_maps(S.h_galpha, ra, n);
   cas_string_maps(S.h_ubeta, rb, n);
-  ScopedBuffers<12> buf(c);
-  std::vector<double> h4(n4), h2(n2);
-
+  auto up = [&](DeviceBuffer& b, const void* src, size_t bytes) {
+    void* p = dev_alloc(c, b, bytes + 16);
+    QDKGB_CUDA(cudaMemcpyAsync(p, src, bytes, cudaMemcpyHostToDevice, c->stream));
+  };
   // ---------------- opposite spin (aabb)
-  if (aabb) {
-    // beta lists per class (i, j): (bI, bJ, s_b) packed bI | bJ << 15 | s << 31
-    std::vector<uint32_t> blist;
-    std::vector<int32_t> bbeg(n2 + 1, 0);
-    for (int j = 0; j < n; ++j)
-      for (int i = 0; i < n; ++i) {
-        const int cls = i + n * j;
-        bbeg[cls] = (int32_t)blist.size();
-        for (int64_t x = 0; x < nb; ++x) {
-          const uint64_t ket = S.h_ubeta[x];
-          if (!((ket >> j) & 1)) continue;
-          if (i == j) {
-            blist.push_back((uint32_t)x | ((uint32_t)x << 15));
-            continue;
-          }
-          if ((ket >> i) & 1) continue;
-          const uint64_t bra = ket ^ (1ull << i) ^ (1ull << j);
-          const int32_t y = rb[bra];
-          if (y < 0) throw Error(QDKGB_ERR_UNSUPPORTED, "RDM: beta strings are not a complete set");
-          const bool neg = cas_sign_odd(ket, (uint32_t)i, (uint32_t)j);
-          blist.push_back((uint32_t)y | ((uint32_t)x << 15) | ((uint32_t)neg << 31));
+  // beta lists per class (i, j): (bI, bJ, s_b) packed bI | bJ << 15 | s << 31
+  std::vector<uint32_t> blist;
+  std::vector<int32_t> bbeg(n2 + 1, 0);
+  for (int j = 0; j < n; ++j)
+    for (int i = 0; i < n; ++i) {
+      const int cls = i + n * j;
+      bbeg[cls] = (int32_t)blist.size();
+      for (int64_t x = 0; x < nb; ++x) {
+        const uint64_t ket = S.h_ubeta[x];
+        if (!((ket >> j) & 1)) continue;
+        if (i == j) {
+          blist.push_back((uint32_t)x | ((uint32_t)x << 15));
+          continue;
         }
+        if ((ket >> i) & 1) continue;
+        const uint64_t bra = ket ^ (1ull << i) ^ (1ull << j);
+        const int32_t y = rb[bra];
+        if (y < 0) throw Error(QDKGB_ERR_UNSUPPORTED, "RDM: beta strings are not a complete set");
+        const bool neg = cas_sign_odd(ket, (uint32_t)i, (uint32_t)j);
+        blist.push_back((uint32_t)y | ((uint32_t)x << 15) | ((uint32_t)neg << 31));
       }
-    bbeg[n2] = (int32_t)blist.size();
-    // work items: lists split to at most the longest off-diagonal length
-    int32_t lmax = 1;
-    for (size_t cl = 0; cl < n2; ++cl)
-      if ((int)(cl % n) != (int)(cl / n)) lmax = std::max(lmax, bbeg[cl + 1] - bbeg[cl]);
-    for (size_t cl = 0; cl < n2; ++cl)
-      if ((int)(cl % n) == (int)(cl / n) && lmax == 1) lmax = std::max(lmax, bbeg[cl + 1] - bbeg[cl]);
-    std::vector<CasItem> items;
-    std::vector<int2> bitems(n2);
-    for (size_t cl = 0; cl < n2; ++cl) {
-      const int32_t len = bbeg[cl + 1] - bbeg[cl];
-      const int parts = std::max(1, (len + lmax - 1) / lmax);
-      bitems[cl].x = (int)items.size();
-      for (int q = 0; q < parts; ++q) {
-        const int32_t b0 = (int32_t)((int64_t)len * q / parts), b1 = (int32_t)((int64_t)len * (q + 1) / parts);
-        items.push_back({(int32_t)cl, bbeg[cl] + b0, b1 - b0});
-      }
-      bitems[cl].y = (int)items.size();
     }
-    const int nitems = (int)items.size();
-    if (nitems > kCasThreads) return false;
+  bbeg[n2] = (int32_t)blist.size();
+  // work items: lists split to at most the longest off-diagonal length
+  int32_t lmax = 1;
+  for (size_t cl = 0; cl < n2; ++cl)
+    if ((int)(cl % n) != (int)(cl / n)) lmax = std::max(lmax, bbeg[cl + 1] - bbeg[cl]);
+  for (size_t cl = 0; cl < n2; ++cl)
+    if ((int)(cl % n) == (int)(cl / n) && lmax == 1) lmax = std::max(lmax, bbeg[cl + 1] - bbeg[cl]);
+  std::vector<CasItem> items;
+  std::vector<int2> bitems(n2);
+  for (size_t cl = 0; cl < n2; ++cl) {
+    const int32_t len = bbeg[cl + 1] - bbeg[cl];
+    const int parts = std::max(1, (len + lmax - 1) / lmax);
+    bitems[cl].x = (int)items.size();
+    for (int q = 0; q < parts; ++q) {
+      const int32_t b0 = (int32_t)((int64_t)len * q / parts), b1 = (int32_t)((int64_t)len * (q + 1) / parts);
+      items.push_back({(int32_t)cl, bbeg[cl] + b0, b1 - b0});
+    }
+    bitems[cl].y = (int)items.size();
+  }
+  const int nitems = (int)items.size();
+  if (nitems <= kCasThreads) {
+    P->ab = true;
+    P->nitems = nitems;
+    P->istride = (nitems + 31) / 32 * 32;
+    P->len = 0;
+    for (const CasItem& i : items) P->len = std::max(P->len, i.len);
+    // transposed, padded with the zero cell
+    std::vector<uint32_t> tl((size_t)P->len * P->istride, (uint32_t)nb | ((uint32_t)nb << 15));
+    for (int i = 0; i < nitems; ++i)
+      for (int e = 0; e < items[i].len; ++e) tl[(size_t)e * P->istride + i] = blist[items[i].begin + e];
     // alpha transitions per class (k, l), k >= l: (gI, gJ, s_a)
     std::vector<uint32_t> atr;
     std::vector<int2> acls, acls_chunks;
@@ -474,56 +597,41 @@ static bool rdms_cas(Context* c, const double* dC, double* aa, double* bb, doubl
         const size_t t1 = atr.size();
         if (t1 == t0) continue;
         acls.push_back({k, l});
+        if (k == l) {
+          acls_chunks.push_back({(int)t0, (int)t1});
+          continue;
+        }
         const int c0 = (int)chunks.size();
         for (size_t q = t0; q < t1; q += kCasChunk)
-          chunks.push_back({(int)acls.size() - 1, (int)q, (int)std::min<size_t>(kCasChunk, t1 - q), 0});
+          chunks.push_back({(int)acls.size() - 1, (int)q, (int)std::min<size_t>(kCasChunk, t1 - q), (int)na});
         acls_chunks.push_back({c0, (int)chunks.size()});
       }
-    double* dG = dev_array<double>(c, buf.b[0], n4);
-    QDKGB_CUDA(cudaMemsetAsync(dG, 0, n4 * 8, c->stream));
-    if (!chunks.empty()) {
-      auto up = [&](DeviceBuffer& b, const void* src, size_t bytes) {
-        void* p = dev_alloc(c, b, bytes + 16);
-        QDKGB_CUDA(cudaMemcpyAsync(p, src, bytes, cudaMemcpyHostToDevice, c->stream));
-        return p;
-      };
-      const uint32_t* d_bl = (const uint32_t*)up(buf.b[1], blist.data(), blist.size() * 4);
-      const CasItem* d_it = (const CasItem*)up(buf.b[2], items.data(), items.size() * sizeof(CasItem));
-      const uint32_t* d_at = (const uint32_t*)up(buf.b[3], atr.data(), atr.size() * 4);
-      const int4* d_ch = (const int4*)up(buf.b[4], chunks.data(), chunks.size() * sizeof(int4));
-      const int2* d_ac = (const int2*)up(buf.b[5], acls.data(), acls.size() * sizeof(int2));
-      const int2* d_acc = (const int2*)up(buf.b[6], acls_chunks.data(), acls_chunks.size() * sizeof(int2));
-      const int2* d_bi = (const int2*)up(buf.b[7], bitems.data(), bitems.size() * sizeof(int2));
-      double* d_part = dev_array<double>(c, buf.b[8], chunks.size() * nitems);
-      const size_t smem = (size_t)2 * nb * 8;
-      set_max_dynamic_smem((const void*)k_rdm_cas_ab, (int)std::max<size_t>(smem, 48 * 1024));
-      k_rdm_cas_ab<<<(unsigned)chunks.size(), kCasThreads, smem, c->stream>>>(nb, dC, d_at, d_ch, d_it, nitems, d_bl,
-                                                                               d_part);
-      QDKGB_CHECK_LAUNCH();
-      const int64_t nred = (int64_t)acls.size() * n2;
-      k_rdm_cas_ab_reduce<<<(unsigned)((nred + 127) / 128), 128, 0, c->stream>>>(n, (int)acls.size(), d_ac, d_acc,
-                                                                                   d_bi, nitems, d_part, dG);
-      QDKGB_CHECK_LAUNCH();
-    }
-    QDKGB_CUDA(cudaMemcpyAsync(h4.data(), dG, n4 * 8, cudaMemcpyDeviceToHost, c->stream));
+    P->nacls = (int)acls.size();
+    P->nchunks = (int)chunks.size();
+    if (chunks.empty()) chunks.push_back({0, 0, 0, (int)na});
+    up(P->bl, tl.data(), tl.size() * 4);
+    up(P->at, atr.data(), atr.size() * 4);
+    up(P->ch, chunks.data(), chunks.size() * sizeof(int4));
+    up(P->ac, acls.data(), acls.size() * sizeof(int2));
+    up(P->acc, acls_chunks.data(), acls_chunks.size() * sizeof(int2));
+    up(P->bi, bitems.data(), bitems.size() * sizeof(int2));
     QDKGB_CUDA(cudaStreamSynchronize(c->stream));
-    for (size_t i = 0; i < n4; ++i) aabb[i] += h4[i];
   }
-
-  // ---------------- same spin (aaaa + aa from alpha pairs, bbbb + bb from beta pairs)
+  // ---------------- same spin: unordered string pairs within a double
+  // excitation, lower rank first, by the lower string
   for (int blk = 0; blk < 2; ++blk) {
-    double* o4 = blk == 0 ? aaaa : bbbb;
-    double* o2 = blk == 0 ? aa : bb;
-    if (!o4 && !o2) continue;
     const std::vector<uint64_t>& strs = blk == 0 ? S.h_galpha : S.h_ubeta;
     const std::vector<int32_t>& rk = blk == 0 ? ra : rb;
-    // unordered string pairs within a double excitation, lower rank first
     std::vector<int2> pairs;
     const int64_t ns = (int64_t)strs.size();
+    std::vector<int> begin(ns + 1);
+    std::vector<int> occ, vir;
     for (int64_t x = 0; x < ns; ++x) {
       const uint64_t s0 = strs[x];
+      begin[x] = (int)pairs.size();
       pairs.push_back({(int)x, (int)x});
-      std::vector<int> occ, vir;
+      occ.clear();
+      vir.clear();
       for (int p = 0; p < n; ++p) ((s0 >> p) & 1 ? occ : vir).push_back(p);
       auto add = [&](uint64_t t) {
         const int32_t y = rk[t];
@@ -538,49 +646,117 @@ static bool rdms_cas(Context* c, const double* dC, double* aa, double* bb, doubl
             for (size_t w = u + 1; w < vir.size(); ++w)
               add(s0 ^ (1ull << occ[a]) ^ (1ull << occ[b2]) ^ (1ull << vir[u]) ^ (1ull << vir[w]));
     }
-    const int64_t np = (int64_t)pairs.size();
-    int2* d_pairs = (int2*)dev_alloc(c, buf.b[9], np * sizeof(int2) + 16);
-    QDKGB_CUDA(cudaMemcpyAsync(d_pairs, pairs.data(), np * sizeof(int2), cudaMemcpyHostToDevice, c->stream));
-    double* d_S = dev_array<double>(c, buf.b[10], np);
-    const double* X = dC;
-    int64_t cols = nb;
-    if (blk == 1) {  // columns of C as rows
-      double* Ct = dev_array<double>(c, buf.b[11], N);
-      transpose_f64(c, dC, Ct, na, nb);
-      X = Ct;
-      cols = na;
-    }
-    k_pair_overlap<<<(unsigned)std::min<int64_t>((np * 32 + 255) / 256, (int64_t)c->sm_count * 64), 256, 0,
-                     c->stream>>>(np, d_pairs, X, cols, d_S);
-    QDKGB_CHECK_LAUNCH();
-    uint64_t* d_str = (uint64_t*)dev_alloc(c, buf.b[1], strs.size() * 8 + 16);
-    QDKGB_CUDA(cudaMemcpyAsync(d_str, strs.data(), strs.size() * 8, cudaMemcpyHostToDevice, c->stream));
-    double* d4 = dev_array<double>(c, buf.b[2], n4);
-    double* d2 = dev_array<double>(c, buf.b[3], n2);
-    QDKGB_CUDA(cudaMemsetAsync(d4, 0, n4 * 8, c->stream));
-    QDKGB_CUDA(cudaMemsetAsync(d2, 0, n2 * 8, c->stream));
-    RdmTarget T;
-    T.block = blk;
-    T.n = n;
-    T.s_lo = 0;
-    T.s_hi = n;
-    T.t4 = d4;
-    T.t2 = d2;
-    T.shared = false;
-    T.with_ordm = true;
-    k_rdm_cas_same_spin<<<(unsigned)std::min<int64_t>((np + 255) / 256, (int64_t)c->sm_count * 16), 256, 0,
-                          c->stream>>>(np, d_pairs, d_str, d_S, T);
-    QDKGB_CHECK_LAUNCH();
+    begin[ns] = (int)pairs.size();
+    RdmPlan::Spin& T = P->spin[blk];
+    T.np = (int64_t)pairs.size();
+    up(T.pairs, pairs.data(), pairs.size() * sizeof(int2));
+    up(T.begin, begin.data(), begin.size() * 4);
+    up(T.str, strs.data(), strs.size() * 8);
     QDKGB_CUDA(cudaStreamSynchronize(c->stream));
-    if (o4) {
-      QDKGB_CUDA(cudaMemcpy(h4.data(), d4, n4 * 8, cudaMemcpyDeviceToHost));
-      for (size_t i = 0; i < n4; ++i) o4[i] += h4[i];
-    }
-    if (o2) {
-      QDKGB_CUDA(cudaMemcpy(h2.data(), d2, n2 * 8, cudaMemcpyDeviceToHost));
-      for (size_t i = 0; i < n2; ++i) o2[i] += h2[i];
-    }
   }
+  return P;
+}
+
+// Returns false (nothing accumulated) when the sweep does not serve the space.
+static bool rdms_cas(Context* c, const double* C, double* aa, double* bb, double* aaaa, double* bbbb, double* aabb) {
+  const DetSpace& S = c->dets;
+  const int n = c->norb;
+  const int64_t na = S.ngroups, nb = S.nbeta, N = na * nb;
+  const size_t n2 = (size_t)n * n, n4 = n2 * n2;
+  RdmPlan* P = nullptr;
+  try {
+    P = rdm_plan(c);
+    if (aabb && !P->ab) return false;
+    double* dC = dev_array<double>(c, P->C, N);
+    QDKGB_CUDA(cudaMemcpyAsync(dC, C, N * 8, cudaMemcpyHostToDevice, c->stream));
+    double* dG = nullptr;
+    if (aabb) {
+      dG = dev_array<double>(c, P->G, n4);
+      QDKGB_CUDA(cudaMemsetAsync(dG, 0, n4 * 8, c->stream));
+      if (P->nacls) {
+        const int rows = P->nchunks + (int)na;  // the chunks' partial sums, then the strings'
+        double* d_part = dev_array<double>(c, P->part, (size_t)rows * P->nitems);
+        double* d_diag = d_part + (size_t)P->nchunks * P->nitems;
+        const bool two = (size_t)4 * (nb + 1) * 8 <= 220 * 1024;
+        const size_t smem = (size_t)(two ? 4 : 2) * (nb + 1) * 8;
+        auto go = [&](auto kern, int64_t blocks, double* out) {
+          if (blocks == 0) return;
+          set_max_dynamic_smem((const void*)kern, (int)std::max<size_t>(smem, 48 * 1024));
+          kern<<<(unsigned)blocks, kCasThreads, smem, c->stream>>>(
+              nb, dC, (const uint32_t*)P->at.ptr, (const int4*)P->ch.ptr, P->nitems, P->istride, P->len,
+              (const uint32_t*)P->bl.ptr, out);
+          QDKGB_CHECK_LAUNCH();
+        };
+        if (two) {
+          go(k_rdm_cas_ab<true, false>, P->nchunks, d_part);
+          go(k_rdm_cas_ab<true, true>, (na + 1) / 2, d_diag);
+        } else {
+          go(k_rdm_cas_ab<false, false>, P->nchunks, d_part);
+          go(k_rdm_cas_ab<false, true>, na, d_diag);
+        }
+        const int64_t nred = (int64_t)P->nacls * n2;
+        k_rdm_cas_ab_reduce<<<(unsigned)((nred * 32 + 127) / 128), 128, 0, c->stream>>>(
+            n, P->nacls, (const int2*)P->ac.ptr, (const int2*)P->acc.ptr, (const int2*)P->bi.ptr, P->nitems, d_part,
+            (const uint32_t*)P->at.ptr, d_diag, dG);
+        QDKGB_CHECK_LAUNCH();
+      }
+    }
+    // same spin (aaaa + aa from alpha pairs, bbbb + bb from beta pairs)
+    double* t4 = dev_array<double>(c, P->t4, 2 * n4);
+    double* t2 = dev_array<double>(c, P->t2, 2 * n2);
+    double* out4[2] = {aaaa, bbbb};
+    double* out2[2] = {aa, bb};
+    for (int blk = 0; blk < 2; ++blk) {
+      if (!out4[blk] && !out2[blk]) continue;
+      RdmPlan::Spin& T = P->spin[blk];
+      double* d_S = dev_array<double>(c, P->S, T.np);
+      const double* X = dC;
+      int64_t rows = na, cols = nb;
+      if (blk == 1) {  // columns of C as rows
+        double* Ct = dev_array<double>(c, P->Ct, N);
+        transpose_f64(c, dC, Ct, na, nb);
+        X = Ct;
+        rows = nb;
+        cols = na;
+      }
+      // the row in shared memory while several CTAs still share an SM
+      const bool staged = cols * 8 <= 56 * 1024;
+      set_max_dynamic_smem((const void*)k_pair_overlap, 56 * 1024);
+      k_pair_overlap<<<(unsigned)rows, 256, staged ? cols * 8 : 0, c->stream>>>(
+          (const int*)T.begin.ptr, (const int2*)T.pairs.ptr, X, cols, staged ? 1 : 0, d_S);
+      QDKGB_CHECK_LAUNCH();
+      QDKGB_CUDA(cudaMemsetAsync(t4 + blk * n4, 0, n4 * 8, c->stream));
+      QDKGB_CUDA(cudaMemsetAsync(t2 + blk * n2, 0, n2 * 8, c->stream));
+      RdmTarget G;
+      G.block = blk;
+      G.n = n;
+      G.s_lo = 0;
+      G.s_hi = n;
+      G.t4 = t4 + blk * n4;
+      G.t2 = t2 + blk * n2;
+      G.shared = false;
+      G.with_ordm = true;
+      k_rdm_cas_same_spin<<<(unsigned)std::min<int64_t>((T.np + 255) / 256, (int64_t)c->sm_count * 16), 256, 0,
+                            c->stream>>>(T.np, (const int2*)T.pairs.ptr, (const uint64_t*)T.str.ptr, d_S, G);
+      QDKGB_CHECK_LAUNCH();
+    }
+    std::vector<double> h4(n4), h2(n2);
+    auto add = [&](double* out, const double* dev, std::vector<double>& h) {
+      if (!out) return;
+      QDKGB_CUDA(cudaMemcpyAsync(h.data(), dev, h.size() * 8, cudaMemcpyDeviceToHost, c->stream));
+      QDKGB_CUDA(cudaStreamSynchronize(c->stream));
+      for (size_t i = 0; i < h.size(); ++i) out[i] += h[i];
+    };
+    add(aabb, dG, h4);
+    for (int blk = 0; blk < 2; ++blk) {
+      add(out4[blk], t4 + blk * n4, h4);
+      add(out2[blk], t2 + blk * n2, h2);
+    }
+  } catch (...) {
+    free_rdm(c);
+    throw;
+  }
+  trim_rdm(c);
   return true;
 }
 
@@ -591,15 +767,15 @@ void rdms_spin_dep(Context* c, const double* C, double* aa, double* bb, double* 
   const int n = c->norb;
   const int64_t N = c->dets.ndets;
   const size_t n2 = (size_t)n * n, n4 = n2 * n2;
-  ScopedBuffers<3> scratch(c);
-  DeviceBuffer &bC = scratch.b[0], &b4 = scratch.b[1], &b2 = scratch.b[2];
-  double* dC = dev_array<double>(c, bC, N);
-  QDKGB_CUDA(cudaMemcpyAsync(dC, C, N * 8, cudaMemcpyHostToDevice, c->stream));
   // QDKGB_RDM_PAIR_WALK=1 keeps complete spaces on the pair walk (a test
   // compares the two paths)
   const char* walk = getenv("QDKGB_RDM_PAIR_WALK");
   const bool force_walk = walk && walk[0] == '1';
-  if (!force_walk && cas_rdm_eligible(c) && rdms_cas(c, dC, aa, bb, aaaa, bbbb, aabb)) return;
+  if (!force_walk && cas_rdm_eligible(c) && rdms_cas(c, C, aa, bb, aaaa, bbbb, aabb)) return;
+  ScopedBuffers<3> scratch(c);
+  DeviceBuffer &bC = scratch.b[0], &b4 = scratch.b[1], &b2 = scratch.b[2];
+  double* dC = dev_array<double>(c, bC, N);
+  QDKGB_CUDA(cudaMemcpyAsync(dC, C, N * 8, cudaMemcpyHostToDevice, c->stream));
   double* d4 = dev_array<double>(c, b4, n4);
   unsigned long long* d2 = dev_array<unsigned long long>(c, b2, 2 * n2);
   RowArgs a = row_args(c, 0.);
