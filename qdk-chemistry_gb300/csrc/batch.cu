@@ -56,49 +56,105 @@ __device__ double bsum(double v, double* red) {
   return t;  // valid in thread 0
 }
 
-// partial[b][chunk][j] = sum over the chunk of A[b][j][i] * w[b][i], j < kk,
-// kk = *kdev + kadd (kdev may be null: kk = kadd).  w is offset by
-// (*kdev) * wk_ld when wk_ld != 0 (the newest column of a stacked basis).
+// Where the sums of a kernel with a CTA per (chunk, instance) end up: each CTA
+// leaves its nv partial sums, and the instance's last CTA adds them in chunk
+// order (deterministic) into out[b * ostride + j], or with Hs into row and
+// column k of the instance's projected matrix (ld m).  count[b] is zero before
+// and after.
+struct BatchSums {
+  double* partial;  // [B][nchunk][KM]
+  int KM;
+  unsigned* count;  // [B]
+  double* out;
+  int64_t ostride;
+  double* Hs;
+  int m;
+};
+__device__ __forceinline__ bool last_chunk(const BatchSums& g, int b) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(g.count + b, 1u) == gridDim.x - 1;
+    if (last) g.count[b] = 0u;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+__device__ __forceinline__ void finish_sums(const BatchSums& g, int b, int nv, int k) {
+  if (!last_chunk(g, b)) return;
+  const int nchunk = gridDim.x;
+  for (int j = threadIdx.x; j < nv; j += blockDim.x) {
+    double s = 0.;
+    for (int c = 0; c < nchunk; ++c) s += __ldcg(g.partial + ((int64_t)b * nchunk + c) * g.KM + j);
+    if (g.Hs) {
+      double* H = g.Hs + (int64_t)b * g.m * g.m;
+      H[k + (int64_t)j * g.m] = s;
+      H[j + (int64_t)k * g.m] = s;
+    } else {
+      g.out[b * g.ostride + j] = s;
+    }
+  }
+}
+
+// out[b][j] = sum over A[b][j][i] * w[b][i], j < kk, kk = *kdev + kadd (kdev
+// may be null: kk = kadd).  w is offset by (*kdev) * wk_ld when wk_ld != 0
+// (the newest column of a stacked basis).  Eight columns at a time: their
+// sums cross the warp with nine FP64 additions instead of forty and the block
+// with one barrier instead of sixteen.  Over the 48 instances of 6e6o, 8e8o
+// and 10e10o a launch takes 9.4 us on average (10.8 column by column) and the
+// separate reduction, 4.7 us, is gone: what is left is the basis from L2.
 __global__ void __launch_bounds__(kBT)
     k_b_multidot(const double* __restrict__ A, int64_t astride, int64_t ld, const int* __restrict__ kdev, int kadd,
-                 const double* __restrict__ w, int64_t wstride, int64_t wk_ld, int64_t n, int nchunk,
-                 double* __restrict__ partial, int KM, const int* __restrict__ mask) {
-  __shared__ double red[33];
+                 const double* __restrict__ w, int64_t wstride, int64_t wk_ld, int64_t n, BatchSums g,
+                 const int* __restrict__ mask) {
+  __shared__ double red[2][kBT / 32][8];
   const int b = blockIdx.y;
   if (mask && !mask[b]) return;
-  const int kk = (kdev ? *kdev : 0) + kadd;
+  const int k0 = kdev ? *kdev : 0, kk = k0 + kadd;
   const int64_t i0 = (int64_t)blockIdx.x * kChunk;
   const double* Ab = A + b * astride;
   const double* wb = w + b * wstride + (wk_ld && kdev ? (int64_t)(*kdev) * wk_ld : 0);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   double wv[kChunk / kBT];
 #pragma unroll
   for (int t = 0; t < kChunk / kBT; ++t) {
     const int64_t i = i0 + threadIdx.x + (int64_t)t * kBT;
     wv[t] = i < n ? wb[i] : 0.;
   }
-  for (int j = 0; j < kk; ++j) {
-    double acc = 0.;
+  double* P = g.partial + ((int64_t)b * gridDim.x + blockIdx.x) * g.KM;
+  for (int j0 = 0, buf = 0; j0 < kk; j0 += 8, buf ^= 1) {
+    double v[8];
 #pragma unroll
-    for (int t = 0; t < kChunk / kBT; ++t) {
-      const int64_t i = i0 + threadIdx.x + (int64_t)t * kBT;
-      if (i < n) acc += Ab[j * ld + i] * wv[t];
+    for (int c = 0; c < 8; ++c) {
+      v[c] = 0.;
+      if (j0 + c >= kk) continue;
+#pragma unroll
+      for (int t = 0; t < kChunk / kBT; ++t) {
+        const int64_t i = i0 + threadIdx.x + (int64_t)t * kBT;
+        if (i < n) v[c] += Ab[(j0 + c) * ld + i] * wv[t];
+      }
     }
-    acc = bsum(acc, red);
-    if (threadIdx.x == 0) partial[((int64_t)b * nchunk + blockIdx.x) * KM + j] = acc;
+#pragma unroll
+    for (int h = 4; h >= 1; h >>= 1) {
+      const bool up = lane & (4 * h);
+#pragma unroll
+      for (int q = 0; q < h; ++q)
+        v[q] = (up ? v[q + h] : v[q]) + __shfl_xor_sync(QDKGB_FULL_MASK, up ? v[q] : v[q + h], 4 * h);
+    }
+    v[0] += __shfl_xor_sync(QDKGB_FULL_MASK, v[0], 2);
+    v[0] += __shfl_xor_sync(QDKGB_FULL_MASK, v[0], 1);
+    if ((lane & 3) == 0) red[buf][wid][((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1)] = v[0];
+    __syncthreads();
+    if (threadIdx.x < 8 && j0 + (int)threadIdx.x < kk) {
+      double t = 0.;
+#pragma unroll
+      for (int q = 0; q < kBT / 32; ++q) t += red[buf][q][threadIdx.x];
+      P[j0 + threadIdx.x] = t;
+    }
   }
-}
-
-// out[b][j] = sum over chunks in order (deterministic)
-__global__ void k_b_reduce(const double* __restrict__ partial, int nchunk, int KM, const int* __restrict__ kdev,
-                           int kadd, double* __restrict__ out, int64_t ostride, const int* __restrict__ mask) {
-  const int b = blockIdx.x;
-  if (mask && !mask[b]) return;
-  const int kk = (kdev ? *kdev : 0) + kadd;
-  for (int j = threadIdx.x; j < kk; j += blockDim.x) {
-    double s = 0.;
-    for (int c = 0; c < nchunk; ++c) s += partial[((int64_t)b * nchunk + c) * KM + j];
-    out[b * ostride + j] = s;
-  }
+  finish_sums(g, b, kk, k0);
 }
 
 // y[b] = (w ? w[b] : 0) + alpha * sum_{j < kk} A[b][j] c[b][j]
@@ -124,7 +180,7 @@ __global__ void __launch_bounds__(kBT)
     k_b_ritz(const double* __restrict__ Vb, const double* __restrict__ AVb, int64_t astride, int64_t ld,
              const int* __restrict__ kdev, const double* __restrict__ yv, int KM, const double* __restrict__ theta,
              double* __restrict__ x, double* __restrict__ xprev, double* __restrict__ ax, double* __restrict__ r,
-             int64_t n, int nchunk, double* __restrict__ partial, const int* __restrict__ mask) {
+             int64_t n, BatchSums g, const int* __restrict__ mask) {
   __shared__ double red[33];
   const int b = blockIdx.y;
   if (mask && !mask[b]) return;
@@ -149,7 +205,8 @@ __global__ void __launch_bounds__(kBT)
     acc += rr * rr;
   }
   acc = bsum(acc, red);
-  if (threadIdx.x == 0) partial[(int64_t)b * nchunk + blockIdx.x] = acc;
+  if (threadIdx.x == 0) g.partial[((int64_t)b * gridDim.x + blockIdx.x) * g.KM] = acc;
+  finish_sums(g, b, 1, 0);
 }
 
 // t = -r / (D - theta), |D - theta| clamped below by min_abs (davidson.hpp:106-113)
@@ -228,15 +285,6 @@ __global__ void k_b_f64_to_col(const double* __restrict__ y, double* __restrict_
     a[i] = y[b * n + i];
 }
 
-// row k of the projected matrix, Hs(k, j) = coef[j], j <= k (lower triangle)
-__global__ void k_b_hsrow(const double* __restrict__ coef, int KM, double* __restrict__ Hs, int m,
-                          const int* __restrict__ kdev, const int* __restrict__ mask) {
-  const int b = blockIdx.x;
-  if (mask && !mask[b]) return;
-  const int k = *kdev;
-  for (int j = threadIdx.x; j <= k; j += blockDim.x) Hs[(int64_t)b * m * m + k + (int64_t)j * m] = coef[(int64_t)b * KM + j];
-}
-
 __global__ void k_b_kinc(int* kdev) { *kdev += 1; }
 
 // second Gram-Schmidt pass where the first removed more than half of |t|^2
@@ -286,8 +334,8 @@ __global__ void k_b_refresh_x(double* __restrict__ x, const double* __restrict__
 // r = ax - theta x (theta = x.ax), AV[b][0] = ax; partial |r|^2
 __global__ void __launch_bounds__(kBT)
     k_b_refresh_res(const double* __restrict__ x, const double* __restrict__ ax, const double* __restrict__ th2,
-                    double* __restrict__ AVb, int64_t astride, double* __restrict__ r, int64_t n, int nchunk,
-                    double* __restrict__ partial, const int* __restrict__ mask) {
+                    double* __restrict__ AVb, int64_t astride, double* __restrict__ r, int64_t n, BatchSums g,
+                    const int* __restrict__ mask) {
   __shared__ double red[33];
   const int b = blockIdx.y;
   if (mask && !mask[b]) return;
@@ -304,14 +352,15 @@ __global__ void __launch_bounds__(kBT)
     acc += rr * rr;
   }
   acc = bsum(acc, red);
-  if (threadIdx.x == 0) partial[(int64_t)b * nchunk + blockIdx.x] = acc;
+  if (threadIdx.x == 0) g.partial[((int64_t)b * gridDim.x + blockIdx.x) * g.KM] = acc;
+  finish_sums(g, b, 1, 0);
 }
 
 // GD+1 restart: partial sums of x.v and v.v for the candidates
 // v = xprev, r, filler (six sums per chunk)
 __global__ void __launch_bounds__(kBT)
     k_b_second_dots(const double* __restrict__ x, const double* __restrict__ xprev, const double* __restrict__ r,
-                    int64_t n, int64_t nstr, const double* __restrict__ flip, int nchunk, double* __restrict__ partial,
+                    int64_t n, int64_t nstr, const double* __restrict__ flip, BatchSums g,
                     const int* __restrict__ mask) {
   __shared__ double red[33];
   const int b = blockIdx.y;
@@ -332,8 +381,9 @@ __global__ void __launch_bounds__(kBT)
   }
   for (int j = 0; j < 6; ++j) {
     const double v = bsum(a[j], red);
-    if (threadIdx.x == 0) partial[((int64_t)b * nchunk + blockIdx.x) * 6 + j] = v;
+    if (threadIdx.x == 0) g.partial[((int64_t)b * gridDim.x + blockIdx.x) * g.KM + j] = v;
   }
+  finish_sums(g, b, 6, 0);
 }
 
 // V[b][1] = (v - (x.v) x) / |.| for the first candidate that keeps a 1e-4
@@ -540,7 +590,7 @@ void casci_batch(Context* ctx, int ninst, const qdkgb_cas_instance* inst, const 
       // every device buffer of the sub-batch, freed on every exit
       struct BufSet {
         Context* c;
-        DeviceBuffer b[40];
+        DeviceBuffer b[42];
         ~BufSet() {
           for (DeviceBuffer& x : b) dev_free(c, x);
         }
@@ -639,7 +689,7 @@ void casci_batch(Context* ctx, int ninst, const qdkgb_cas_instance* inst, const 
                    &by = bs.b[22], &bev = bs.b[23], &bth = bs.b[24], &bco = bs.b[25], &bpart = bs.b[26],
                    &bsc = bs.b[27], &bsc2 = bs.b[28], &bflip = bs.b[29], &bint = bs.b[30], &bidx = bs.b[31],
                    &blt = bs.b[32], &ben = bs.b[33], &bres = bs.b[34], &bxp = bs.b[37], &bw0 = bs.b[38],
-                   &bn2 = bs.b[39];
+                   &bn2 = bs.b[39], &bcnt = bs.b[40], &beig = bs.b[41];
       const int64_t astride = (int64_t)m * N;
       double* Vb = dev_array<double>(cc, bV, (size_t)B * astride);
       double* AVb = dev_array<double>(cc, bAV, (size_t)B * astride);
@@ -657,7 +707,8 @@ void casci_batch(Context* ctx, int ninst, const qdkgb_cas_instance* inst, const 
       double* yv = dev_array<double>(cc, bev, (size_t)B * KM);
       double* theta = dev_array<double>(cc, bth, (size_t)B);
       double* coef = dev_array<double>(cc, bco, (size_t)B * KM);
-      double* partial = dev_array<double>(cc, bpart, (size_t)B * nchunk * std::max(KM, 6));
+      const int PM = std::max(KM, 6);
+      double* partial = dev_array<double>(cc, bpart, (size_t)B * nchunk * PM);
       double* sc = dev_array<double>(cc, bsc, (size_t)B * 6);    // per-instance scalars
       double* sc2 = dev_array<double>(cc, bsc2, (size_t)B * 2);  // second scalar
       double* flip = dev_array<double>(cc, bflip, (size_t)B);
@@ -674,6 +725,13 @@ void casci_batch(Context* ctx, int ninst, const qdkgb_cas_instance* inst, const 
       int64_t* idx = dev_array<int64_t>(cc, bidx, (size_t)B);
       double* w0 = dev_array<double>(cc, bw0, (size_t)B);  // |t|^2 before the first Gram-Schmidt pass
       int* need2 = dev_array<int>(cc, bn2, (size_t)B);     // instances that take the second pass
+      unsigned* count = dev_array<unsigned>(cc, bcnt, (size_t)B);
+      // the projected problems' states from size to size
+      unsigned char* eig = (unsigned char*)dev_alloc(cc, beig, (size_t)B * eig_warm_bytes(m));
+      QDKGB_CUDA(cudaMemsetAsync(count, 0, (size_t)B * 4, s0));
+      QDKGB_CUDA(cudaMemsetAsync(eig, 0, (size_t)B * eig_warm_bytes(m), s0));
+      auto sums = [&](double* out, int64_t ostride) { return BatchSums{partial, PM, count, out, ostride, nullptr, m}; };
+      const BatchSums to_row{partial, PM, count, nullptr, 0, Hs, m};
       QDKGB_CUDA(cudaMemsetAsync(ints, 0, ((size_t)5 * B + 8) * sizeof(int), s0));
       QDKGB_CUDA(cudaMemsetAsync(Hs, 0, (size_t)B * m * m * 8, s0));
       // guess and its spin-flip sector (kept by the FP64 iteration; FP32
@@ -705,9 +763,7 @@ void casci_batch(Context* ctx, int ninst, const qdkgb_cas_instance* inst, const 
       // the previous Ritz vector orthogonalised against x, also multiplied
       // in full precision) instead of x alone
       auto refresh = [&](bool gd) {
-        k_b_multidot<<<gc, kBT, 0, s0>>>(x, N, N, nullptr, 1, x, N, 0, N, nchunk, partial, KM, notdone);
-        QDKGB_CHECK_LAUNCH();
-        k_b_reduce<<<B, 32, 0, s0>>>(partial, nchunk, KM, nullptr, 1, sc, 6, notdone);
+        k_b_multidot<<<gc, kBT, 0, s0>>>(x, N, N, nullptr, 1, x, N, 0, N, sums(sc, 6), notdone);
         QDKGB_CHECK_LAUNCH();
         k_b_refresh_x<<<gv, kBT, 0, s0>>>(x, sc, 6, Vb, astride, xh, xl, N, notdone);
         QDKGB_CHECK_LAUNCH();
@@ -721,9 +777,7 @@ void casci_batch(Context* ctx, int ninst, const qdkgb_cas_instance* inst, const 
             k_b_flip<<<gv, kBT, 0, s0>>>(r, S.nbeta, flip, notdone);
             QDKGB_CHECK_LAUNCH();
           }
-          k_b_second_dots<<<gc, kBT, 0, s0>>>(x, xprev, r, N, S.nbeta, fl, nchunk, partial, notdone);
-          QDKGB_CHECK_LAUNCH();
-          k_b_reduce<<<B, 32, 0, s0>>>(partial, nchunk, 6, nullptr, 6, sc, 6, notdone);
+          k_b_second_dots<<<gc, kBT, 0, s0>>>(x, xprev, r, N, S.nbeta, fl, sums(sc, 6), notdone);
           QDKGB_CHECK_LAUNCH();
           k_b_second_set<<<gv, kBT, 0, s0>>>(x, xprev, r, sc, Vb, astride, ld, t32, s32, N, S.nbeta, fl, notdone);
           QDKGB_CHECK_LAUNCH();
@@ -737,13 +791,9 @@ void casci_batch(Context* ctx, int ninst, const qdkgb_cas_instance* inst, const 
         }
         if (mixed) slab_sigma_batch(cc, 2, B, notdone, hi, lo, xh, xl, yfull);
         else slab_sigma_batch(cc, 1, B, notdone, val, nullptr, x, nullptr, yfull);
-        k_b_multidot<<<gc, kBT, 0, s0>>>(x, N, N, nullptr, 1, yfull, N, 0, N, nchunk, partial, KM, notdone);
+        k_b_multidot<<<gc, kBT, 0, s0>>>(x, N, N, nullptr, 1, yfull, N, 0, N, sums(sc2, 2), notdone);
         QDKGB_CHECK_LAUNCH();
-        k_b_reduce<<<B, 32, 0, s0>>>(partial, nchunk, KM, nullptr, 1, sc2, 2, notdone);
-        QDKGB_CHECK_LAUNCH();
-        k_b_refresh_res<<<gc, kBT, 0, s0>>>(x, yfull, sc2, AVb, astride, r, N, nchunk, partial, notdone);
-        QDKGB_CHECK_LAUNCH();
-        k_b_reduce<<<B, 32, 0, s0>>>(partial, nchunk, 1, nullptr, 1, sc, 6, notdone);
+        k_b_refresh_res<<<gc, kBT, 0, s0>>>(x, yfull, sc2, AVb, astride, r, N, sums(sc, 6), notdone);
         QDKGB_CHECK_LAUNCH();
         k_b_check<<<1, 1024, 0, s0>>>(B, sc2, sc, 6, st.res_tol, notdone, act, nref, last_true, theta, energy, Hs, m,
                                       kdev, nact, resid);
@@ -752,17 +802,13 @@ void casci_batch(Context* ctx, int ninst, const qdkgb_cas_instance* inst, const 
           k_b_copy_col<<<gv, kBT, 0, s0>>>(ax, AVb, astride, ld, 1, N, act);
           QDKGB_CHECK_LAUNCH();
           // row 1 of the projected matrix (kdev = 1 after the check), then k = 2
-          k_b_multidot<<<gc, kBT, 0, s0>>>(AVb, astride, ld, kdev, 1, Vb, astride, ld, N, nchunk, partial, KM, act);
-          QDKGB_CHECK_LAUNCH();
-          k_b_reduce<<<B, 64, 0, s0>>>(partial, nchunk, KM, kdev, 1, coef, KM, act);
-          QDKGB_CHECK_LAUNCH();
-          k_b_hsrow<<<B, 64, 0, s0>>>(coef, KM, Hs, m, kdev, act);
+          k_b_multidot<<<gc, kBT, 0, s0>>>(AVb, astride, ld, kdev, 1, Vb, astride, ld, N, to_row, act);
           QDKGB_CHECK_LAUNCH();
           k_b_kinc<<<1, 1, 0, s0>>>(kdev);
           QDKGB_CHECK_LAUNCH();
-          lowest_eig_batch(s0, B, kdev, 0, m, Hs, m, (int64_t)m * m, theta, yv, KM, act);
-          k_b_ritz<<<gc, kBT, 0, s0>>>(Vb, AVb, astride, ld, kdev, yv, KM, theta, x, xprev, ax, r, N, nchunk, partial,
-                                       act);
+          lowest_eig_batch(s0, B, kdev, 0, m, Hs, m, (int64_t)m * m, theta, yv, KM, act, eig, true);
+          k_b_ritz<<<gc, kBT, 0, s0>>>(Vb, AVb, astride, ld, kdev, yv, KM, theta, x, xprev, ax, r, N, sums(sc, 2),
+                                     act);
           QDKGB_CHECK_LAUNCH();
         }
       };
@@ -779,17 +825,13 @@ void casci_batch(Context* ctx, int ninst, const qdkgb_cas_instance* inst, const 
         // instances whose first pass removed more than half of |t|^2 (the
         // Daniel-Gragg-Kaufman-Stewart test, as in the single solve)
         auto gs_pass = [&](const int* mask) {
-          k_b_multidot<<<gc, kBT, 0, s0>>>(Vb, astride, ld, kdev, 0, t, N, 0, N, nchunk, partial, KM, mask);
-          QDKGB_CHECK_LAUNCH();
-          k_b_reduce<<<B, 64, 0, s0>>>(partial, nchunk, KM, kdev, 0, coef, KM, mask);
+          k_b_multidot<<<gc, kBT, 0, s0>>>(Vb, astride, ld, kdev, 0, t, N, 0, N, sums(coef, KM), mask);
           QDKGB_CHECK_LAUNCH();
           k_b_gemv<<<gv, kBT, 0, s0>>>(Vb, astride, ld, kdev, 0, coef, KM, -1., t, t, N, N, mask);
           QDKGB_CHECK_LAUNCH();
         };
         auto norm2 = [&](double* out, int ostride, const int* mask) {
-          k_b_multidot<<<gc, kBT, 0, s0>>>(t, N, N, nullptr, 1, t, N, 0, N, nchunk, partial, KM, mask);
-          QDKGB_CHECK_LAUNCH();
-          k_b_reduce<<<B, 32, 0, s0>>>(partial, nchunk, KM, nullptr, 1, out, ostride, mask);
+          k_b_multidot<<<gc, kBT, 0, s0>>>(t, N, N, nullptr, 1, t, N, 0, N, sums(out, ostride), mask);
           QDKGB_CHECK_LAUNCH();
         };
         if (mixed) {
@@ -821,19 +863,13 @@ void casci_batch(Context* ctx, int ninst, const qdkgb_cas_instance* inst, const 
         // projected row k: Hs(k, j) = AV[j] . V[k], j <= k - the older (more
         // accurate) product of each pair: the exact AV[0] couples the new
         // direction to the refreshed vector
-        k_b_multidot<<<gc, kBT, 0, s0>>>(AVb, astride, ld, kdev, 1, Vb, astride, ld, N, nchunk, partial, KM, act);
-        QDKGB_CHECK_LAUNCH();
-        k_b_reduce<<<B, 64, 0, s0>>>(partial, nchunk, KM, kdev, 1, coef, KM, act);
-        QDKGB_CHECK_LAUNCH();
-        k_b_hsrow<<<B, 64, 0, s0>>>(coef, KM, Hs, m, kdev, act);
+        k_b_multidot<<<gc, kBT, 0, s0>>>(AVb, astride, ld, kdev, 1, Vb, astride, ld, N, to_row, act);
         QDKGB_CHECK_LAUNCH();
         k_b_kinc<<<1, 1, 0, s0>>>(kdev);
         QDKGB_CHECK_LAUNCH();
-        lowest_eig_batch(s0, B, kdev, 0, m, Hs, m, (int64_t)m * m, theta, yv, KM, act);
-        k_b_ritz<<<gc, kBT, 0, s0>>>(Vb, AVb, astride, ld, kdev, yv, KM, theta, x, xprev, ax, r, N, nchunk, partial,
+        lowest_eig_batch(s0, B, kdev, 0, m, Hs, m, (int64_t)m * m, theta, yv, KM, act, eig, false);
+        k_b_ritz<<<gc, kBT, 0, s0>>>(Vb, AVb, astride, ld, kdev, yv, KM, theta, x, xprev, ax, r, N, sums(sc, 2),
                                      act);
-        QDKGB_CHECK_LAUNCH();
-        k_b_reduce<<<B, 32, 0, s0>>>(partial, nchunk, 1, nullptr, 1, sc, 2, act);
         QDKGB_CHECK_LAUNCH();
         k_b_wait<<<1, 1024, 0, s0>>>(B, sc, last_true, 1e-4, kdev, m, act, nact);
         QDKGB_CHECK_LAUNCH();

@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <cstddef>
 #include <vector>
 
 #include "common.cuh"
@@ -831,23 +832,39 @@ __global__ void __launch_bounds__(kEigThreads) k_lowest_eig_next(int k, const do
 }
 
 // One CTA per instance of a batch: the lowest pair of the leading k x k block
-// of Hs[b] (k = *kdev + kadd, matrices hstride apart, ld ldh); CTAs of
-// inactive instances leave at once.
+// of Hs[b] (k = *kdev + kadd, matrices hstride apart, ld ldh, full), from the
+// state of the size before where there is one (26.7 us a launch over a batch's
+// sizes up to 30, 41.6 from scratch); CTAs of inactive instances leave at once.
 __global__ void __launch_bounds__(kEigThreads)
     k_lowest_eig_batch(const int* __restrict__ kdev, int kadd, const double* __restrict__ Hs, int ldh,
-                       int64_t hstride, double* eval, double* evec, int64_t estride, const int* __restrict__ active) {
+                       int64_t hstride, double* eval, double* evec, int64_t estride, const int* __restrict__ active,
+                       unsigned char* states, int64_t sstride, int fresh) {
   const int b = blockIdx.x;
   if (active && !active[b]) return;
   const int k = *kdev + kadd;
-  lowest_eig_cta(k, Hs + b * hstride, ldh, nullptr, 1, eval + b, evec + b * estride);
+  if (!states) {
+    lowest_eig_cta(k, Hs + b * hstride, ldh, nullptr, 1, eval + b, evec + b * estride);
+    return;
+  }
+  EigWarm* st = (EigWarm*)(states + b * sstride);
+  if (fresh) {
+    if (threadIdx.x == 0) st->k = st->kt = 0;
+    __syncthreads();
+  }
+  lowest_eig_next_cta(k, Hs + b * hstride, ldh, nullptr, eval + b, evec + b * estride, st);
+}
+
+size_t eig_warm_bytes(int kmax) {
+  return (offsetof(EigWarm, P) + (size_t)kmax * kmax * sizeof(float) + 15) & ~(size_t)15;
 }
 
 void lowest_eig_batch(cudaStream_t st, int B, const int* kdev, int kadd, int kmax, const double* Hs, int ldh,
-                      int64_t hstride, double* eval, double* evec, int64_t estride, const int* active) {
+                      int64_t hstride, double* eval, double* evec, int64_t estride, const int* active,
+                      unsigned char* states, bool fresh) {
   if (kmax > kEigSmemK) throw Error(QDKGB_ERR_INVALID, "batched subspace larger than the shared-memory eigensolver");
   set_max_dynamic_smem((const void*)k_lowest_eig_batch, (int)kEigDynSmemMax);
-  k_lowest_eig_batch<<<B, kEigThreads, eig_dyn_smem(kmax), st>>>(kdev, kadd, Hs, ldh, hstride, eval, evec, estride,
-                                                                 active);
+  k_lowest_eig_batch<<<B, kEigThreads, std::max(eig_dyn_smem(kmax), eig_warm_smem(kmax)), st>>>(
+      kdev, kadd, Hs, ldh, hstride, eval, evec, estride, active, states, (int64_t)eig_warm_bytes(kmax), fresh ? 1 : 0);
   QDKGB_CHECK_LAUNCH();
 }
 

@@ -245,8 +245,12 @@ void batch_solve_persistent(Context* cc, Context* owner, const BatchShapeJob& jo
 // grow.hpp:196-199), intermediates rebuilt
 void natural_orbitals(int n, const std::vector<double>& ordm, std::vector<double>& C);
 void rotate_integrals(Context* c, const std::vector<double>& C);
+// states: eig_warm_bytes(kmax) bytes per instance, zero before the first call
+// (null: every size from scratch); fresh: another matrix than the last one's.
+size_t eig_warm_bytes(int kmax);
 void lowest_eig_batch(cudaStream_t st, int B, const int* kdev, int kadd, int kmax, const double* Hs, int ldh,
-                      int64_t hstride, double* eval, double* evec, int64_t estride, const int* active);
+                      int64_t hstride, double* eval, double* evec, int64_t estride, const int* active,
+                      unsigned char* states, bool fresh);
 void slab_emit_batch(Context* c, int B, const Integrals* d_ints, const double* diag_raw, int storage, double* val,
                      float* hi, float* lo, double thresh);
 void slab_reserve_batch(Context* c, int B);

@@ -76,7 +76,7 @@ struct EigWarm {
   int k, kt;
   double sigma, theta, scale, gap;  // gap: to the next eigenvalue, when P was made
   double x[kEigWarmMaxK];
-  float P[kEigWarmMaxK * kEigWarmMaxK];  // leading dimension k
+  float P[kEigWarmMaxK * kEigWarmMaxK];  // leading dimension k; shorter where sizes stop below (eig_warm_bytes)
 };
 
 static __device__ void lowest_eig_cta(int k, const double* __restrict__ H, int ldh, double* gA, int nev, double* eval,
