@@ -4,11 +4,11 @@
 // 93-297 and the fast diagonals of src/macis/hamiltonian_generator/
 // fast_diagonals.ipp:52-127).
 //
-// GPU design: one warp per core determinant P enumerates every single and
-// double excitation Q of P as one flat index space (alpha singles, beta
-// singles, alpha-alpha, beta-beta, alpha-beta doubles), evaluates c_P <Q|H|P>
-// and the fast diagonal E0 - H_QQ exactly as the reference does, drops
-// |c h| < h_el_tol, and accumulates into an open-addressing hash table keyed by
+// GPU design: a few CTAs per core determinant P enumerate every single and
+// double excitation Q of P by rows (one beta single, or one pair of occupied
+// orbitals, against all its partners), evaluate c_P <Q|H|P>
+// and the fast diagonal E0 - H_QQ exactly as the reference does, drop
+// |c h| < h_el_tol, and accumulate into an open-addressing hash table keyed by
 // the full (alpha, beta) pair (128-bit atomicCAS, then exact fixed-point
 // integer atomics of c h; see Table below).  That replaces the reference's
 // constraint partitioning plus sort-and-accumulate: every Q's contributions
@@ -64,49 +64,86 @@ constexpr long long kHdEmpty = (long long)0x8000000000000000ULL;
 constexpr double kFixHi = 4294967296.0;               // 2^32
 constexpr double kFixLo = 75557863725914323419136.0;  // 2^76
 
+// A slot's key and sums share one 32-byte sector: a contribution touches two
+// sectors at random (this and hd) instead of three.
+struct __align__(32) Slot {
+  u128 key;
+  long long hi, lo;
+};
 struct Table {
-  u128* keys;
-  long long* acc;  // 2 words per slot (hi, lo)
-  long long* hd;   // bit pattern of E0 - H_QQ, or kCoreMark
-  uint64_t mask;
+  Slot* slot;
+  long long* hd;  // bit pattern of E0 - H_QQ, or kCoreMark
+  uint64_t cap;   // slots (any number: the hash is scaled to it)
   int* err;  // set when a probe sequence runs past kMaxProbe (the table is too full): the pass is redone larger
 };
 constexpr uint64_t kMaxProbe = 4096;
 
 __device__ __forceinline__ double table_sum(const Table& t, uint64_t i) {
-  return (double)t.acc[2 * i] * (1.0 / kFixHi) + (double)t.acc[2 * i + 1] * (1.0 / kFixLo);
+  return (double)t.slot[i].hi * (1.0 / kFixHi) + (double)t.slot[i].lo * (1.0 / kFixLo);
 }
 __device__ __forceinline__ bool table_core(const Table& t, uint64_t i) { return t.hd[i] == kCoreMark; }
 
-// slot of (qa, qb), inserting the key; -1 when the probe limit is reached
-__device__ __forceinline__ int64_t table_slot(const Table& t, uint64_t qa, uint64_t qb) {
-  const u128 key = ((u128)qb << 64) | (u128)qa;
-  uint64_t h = mix64(qa * 0x9e3779b97f4a7c15ULL ^ mix64(qb)) & t.mask;
-  for (uint64_t probe = 0; probe <= t.mask && probe < kMaxProbe; ++probe) {
-    const u128 old = atomicCAS(t.keys + h, kEmpty, key);
-    if (old == kEmpty || old == key) return (int64_t)h;
-    h = (h + 1) & t.mask;
+// |x| as an ordered integer: comparisons off the FP64 pipe
+__device__ __forceinline__ uint64_t magnitude(double x) {
+  return (uint64_t)__double_as_longlong(x) & 0x7fffffffffffffffULL;
+}
+constexpr uint64_t kBits2p19 = (uint64_t)(1023 + 19) << 52, kBits2p20 = (uint64_t)(1023 + 20) << 52;
+constexpr uint64_t kBitsInf = (uint64_t)2047 << 52;
+
+__device__ __forceinline__ u128 table_key(uint64_t qa, uint64_t qb) { return ((u128)qb << 64) | (u128)qa; }
+__device__ __forceinline__ uint64_t table_home(const Table& t, uint64_t qa, uint64_t qb) {
+  return __umul64hi(mix64(qa * 0x9e3779b97f4a7c15ULL ^ mix64(qb)), t.cap);
+}
+// the key's slot, inserted if need be, when its home h held `old` before an
+// exchange; -1 when the probe limit is reached
+__device__ __forceinline__ int64_t table_slot(const Table& t, u128 key, uint64_t h, u128 old) {
+  for (uint64_t probe = 1; old != kEmpty && old != key; ++probe) {
+    if (probe >= t.cap || probe >= kMaxProbe) {
+      *t.err = 1;
+      return -1;
+    }
+    if (++h == t.cap) h = 0;
+    old = atomicCAS(&t.slot[h].key, kEmpty, key);
   }
-  *t.err = 1;
-  return -1;
+  return (int64_t)h;
 }
 
-__device__ __forceinline__ void table_add(const Table& t, uint64_t qa, uint64_t qb, double ch, double hd) {
-  const int64_t h = table_slot(t, qa, qb);
+// Adds ch to the target's sum and meets its diagonal with diag(), which is
+// worked out while the exchange at the target's home slot is under way.
+template <class Diag>
+__device__ __forceinline__ void table_add(const Table& t, uint64_t qa, uint64_t qb, double ch, Diag diag) {
+  const u128 key = table_key(qa, qb);
+  const uint64_t home = table_home(t, qa, qb);
+  const u128 old = atomicCAS(&t.slot[home].key, kEmpty, key);
+  const double hd = diag();
+  // Adding 1.5 x 2^(52 - s) rounds to units of 2^-s (to even, as rint does)
+  // and leaves the integer in the low bits: four FP64 operations instead of
+  // two roundings, two conversions and their scalings.
+  constexpr double kHiM = 1572864.0, kLoM = 6755399441055744.0;  // 1.5 x 2^20, 1.5 x 2^52
+  const double t1 = __dadd_rn(ch, kHiM);
+  const double rest = __dsub_rn(ch, __dsub_rn(t1, kHiM));
+  long long hi = __double_as_longlong(t1) - __double_as_longlong(kHiM);
+  long long lo = __double_as_longlong(__fma_rn(rest, kFixLo, kLoM)) - __double_as_longlong(kLoM);
+  const int64_t h = table_slot(t, key, home, old);
   if (h < 0) return;
-  if (!(fabs(ch) < 1048576.0)) {  // outside the fixed-point range (or not finite)
-    *t.err = 2;
-    return;
+  if (magnitude(ch) >= kBits2p19) {
+    if (magnitude(ch) >= kBits2p20) {  // outside the fixed-point range (or not finite)
+      *t.err = 2;
+      return;
+    }
+    const double h1 = rint(ch * kFixHi);
+    hi = (long long)h1;
+    lo = (long long)rint((ch - h1 * (1.0 / kFixHi)) * kFixLo);
   }
-  const double hi = rint(ch * kFixHi);
-  const double lo = rint((ch - hi * (1.0 / kFixHi)) * kFixLo);
-  atomicAdd((unsigned long long*)t.acc + 2 * h, (unsigned long long)(long long)hi);
-  atomicAdd((unsigned long long*)t.acc + 2 * h + 1, (unsigned long long)(long long)lo);
+  atomicAdd((unsigned long long*)&t.slot[h].hi, (unsigned long long)hi);
+  atomicAdd((unsigned long long*)&t.slot[h].lo, (unsigned long long)lo);
   atomicMax(t.hd + h, (long long)__double_as_longlong(hd));
 }
 
 __device__ __forceinline__ void table_add_core(const Table& t, uint64_t qa, uint64_t qb) {
-  const int64_t h = table_slot(t, qa, qb);
+  const u128 key = table_key(qa, qb);
+  const uint64_t home = table_home(t, qa, qb);
+  const int64_t h = table_slot(t, key, home, atomicCAS(&t.slot[home].key, kEmpty, key));
   if (h >= 0) atomicMax(t.hd + h, kCoreMark);
 }
 
@@ -122,6 +159,12 @@ struct CoreArgs {
   Table T;
   uint32_t npass = 1, pass = 0;  // targets whose part_of() == pass are inserted (npass > 1: PT2 passes)
   bool just_singles = false;     // the search's just_singles: single excitations only
+  int nslice = 1;                // CTAs per core determinant
+  // |x| >= h_el_tol
+  __device__ __forceinline__ bool keeps(double x) const {
+    const uint64_t m = magnitude(x);
+    return (h_el_tol <= 0. || m >= (uint64_t)__double_as_longlong(h_el_tol)) && m <= kBitsInf && h_el_tol == h_el_tol;
+  }
 };
 
 // part of the target space of a determinant in a split into npass passes (a
@@ -130,176 +173,12 @@ __device__ __forceinline__ uint32_t part_of(uint64_t qa, uint64_t qb, uint32_t n
   return (uint32_t)(mix64(qb * 0x9e3779b97f4a7c15ULL ^ mix64(qa + 0x632be59bd9b4e019ULL)) % npass);
 }
 
-// (i, j) with i < j from a pair index p = j (j - 1) / 2 + i
-__device__ __forceinline__ void pair_of(int p, int& i, int& j) {
-  int jj = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)p)) * 0.5f);
-  while (jj * (jj - 1) / 2 > p) --jj;
-  while ((jj + 1) * jj / 2 <= p) ++jj;
-  j = jj;
-  i = p - jj * (jj - 1) / 2;
-}
-
-struct WarpSm {
-  double ea[kMaxOrb], eb[kMaxOrb];
-  uint8_t oa[kMaxOrb], va[kMaxOrb], ob[kMaxOrb], vb[kMaxOrb];
-};
-
 __device__ __forceinline__ double G2at(const Integrals& I, uint32_t p, uint32_t q) {
   return ld(I.G2 + p + (size_t)I.n * q);
 }
 __device__ __forceinline__ double V2at(const Integrals& I, uint32_t p, uint32_t q) {
   return ld(I.V2 + p + (size_t)I.n * q);
 }
-// single_excitation_sign(state, a, i) as a double (+1 / -1)
-__device__ __forceinline__ double sgn(uint64_t state, uint32_t a, uint32_t i) {
-  return excitation_sign_odd(state, a, i) ? -1. : 1.;
-}
-
-__global__ void __launch_bounds__(kAsciWarps * 32) k_asci_enum(CoreArgs A) {
-  __shared__ WarpSm wsm[kAsciWarps];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  WarpSm& s = wsm[w];
-  const Integrals& I = A.I;
-  const int n = A.n;
-  const uint64_t full = (n == 64) ? ~0ull : ((1ull << n) - 1ull);
-  for (int64_t ip = (int64_t)blockIdx.x * kAsciWarps + w; ip < A.ncore; ip += (int64_t)gridDim.x * kAsciWarps) {
-    const uint64_t Pa = A.ca[ip], Pb = A.cb[ip];
-    const double c = A.cc[ip];
-    const int ka = popc64(Pa), kb = popc64(Pb), na_v = n - ka, nb_v = n - kb;
-    // occupied / virtual lists and orbital energies (single_orbital_ens, fast_diagonals.ipp:30-50)
-    if (lane == 0) {
-      int x = 0, y = 0, u = 0, v = 0;
-      for (int p = 0; p < n; ++p) {
-        if ((Pa >> p) & 1)
-          s.oa[x++] = p;
-        else
-          s.va[y++] = p;
-        if ((Pb >> p) & 1)
-          s.ob[u++] = p;
-        else
-          s.vb[v++] = p;
-      }
-    }
-    for (int i = lane; i < n; i += 32) {
-      double e = ld(I.T + i + (size_t)n * i);
-      for (uint64_t m = Pa; m; m &= m - 1) {
-        const uint32_t q = low_bit(m);
-        e += G2at(I, i, q) + G2at(I, q, i);
-      }
-      e -= G2at(I, i, i);
-      for (uint64_t m = Pb; m; m &= m - 1) e += V2at(I, i, low_bit(m));
-      s.ea[i] = e;
-      double f = ld(I.T + i + (size_t)n * i);
-      for (uint64_t m = Pb; m; m &= m - 1) {
-        const uint32_t q = low_bit(m);
-        f += G2at(I, i, q) + G2at(I, q, i);
-      }
-      f -= G2at(I, i, i);
-      for (uint64_t m = Pa; m; m &= m - 1) f += V2at(I, i, low_bit(m));
-      s.eb[i] = f;
-    }
-    double hdiag = 0.;
-    if (lane == 0) hdiag = me_diag(I, Pa, Pb);
-    hdiag = __shfl_sync(QDKGB_FULL_MASK, hdiag, 0);
-    __syncwarp();
-    // the core determinant itself: infinite score (removed later)
-    if (lane == 0 && (A.npass == 1 || part_of(Pa, Pb, A.npass) == A.pass)) table_add_core(A.T, Pa, Pb);
-    const int64_t nsa = (int64_t)ka * na_v, nsb = (int64_t)kb * nb_v;
-    const int64_t pa_o = (int64_t)ka * (ka - 1) / 2, pa_v = (int64_t)na_v * (na_v - 1) / 2;
-    const int64_t pb_o = (int64_t)kb * (kb - 1) / 2, pb_v = (int64_t)nb_v * (nb_v - 1) / 2;
-    const int64_t nda = pa_o * pa_v, ndb = pb_o * pb_v, nab = nsa * nsb;
-    const int64_t total = A.just_singles ? nsa + nsb : nsa + nsb + nda + ndb + nab;
-    for (int64_t e = lane; e < total; e += 32) {
-      double ch = 0., hd = 0.;
-      uint64_t qa = Pa, qb = Pb;
-      bool ok = false;
-      int64_t x = e;
-      if (x < nsa + nsb) {
-        // append_singles_asci_contributions (determinant_contributions.hpp:93-133)
-        const bool alpha = x < nsa;
-        if (!alpha) x -= nsa;
-        const int nv = alpha ? na_v : nb_v;
-        const uint32_t i = alpha ? s.oa[x / nv] : s.ob[x / nv];
-        const uint32_t a = alpha ? s.va[x % nv] : s.vb[x % nv];
-        const uint64_t same = alpha ? Pa : Pb, other = alpha ? Pb : Pa;
-        const size_t nn = (size_t)n;
-        double h = ld(I.T + a + nn * i);
-        const double* G = I.G_red + nn * (a + nn * i);
-        const double* Vr = I.V_red + nn * (a + nn * i);
-        for (uint64_t m = same; m; m &= m - 1) h += ld(G + low_bit(m));
-        for (uint64_t m = other; m; m &= m - 1) h += ld(Vr + low_bit(m));
-        if (fabs(c * h) >= A.h_el_tol) {
-          h *= sgn(same, a, i);
-          const double* eps = alpha ? s.ea : s.eb;
-          const double hdq = hdiag + eps[a] - eps[i] - G2at(I, a, i) - G2at(I, i, a);
-          const uint64_t ex = (same ^ (1ull << i)) | (1ull << a);
-          if (alpha)
-            qa = ex;
-          else
-            qb = ex;
-          ch = c * h;
-          hd = A.E0 - hdq;
-          ok = true;
-        }
-      } else if ((x -= nsa + nsb) < nda + ndb) {
-        // append_ss_doubles_asci_contributions (determinant_contributions.hpp:149-210)
-        const bool alpha = x < nda;
-        if (!alpha) x -= nda;
-        const int64_t pv = alpha ? pa_v : pb_v;
-        int ii, jj, aa, bb;
-        pair_of((int)(x / pv), ii, jj);
-        pair_of((int)(x % pv), aa, bb);
-        const uint8_t* occ = alpha ? s.oa : s.ob;
-        const uint8_t* vir = alpha ? s.va : s.vb;
-        const uint32_t i = occ[ii], j = occ[jj], a = vir[aa], b = vir[bb];
-        const double Gv = Vat(I, b, j, a, i) - Vat(I, b, i, a, j);
-        if (fabs(c * Gv) >= A.h_el_tol) {
-          const uint64_t same = alpha ? Pa : Pb;
-          const uint64_t fullex = (1ull << i) | (1ull << j) | (1ull << a) | (1ull << b);
-          const uint64_t ex = same ^ fullex;
-          // doubles_sign(state_same, ex_det, full_ex): bra = P, ket = Q
-          SingleEx s1 = single_ex(same, ex, fullex);
-          const uint64_t f1 = (1ull << s1.o) | (1ull << s1.v);
-          SingleEx s2 = single_ex(same, ex ^ f1, fullex ^ f1);
-          const double h = (s1.neg != s2.neg) ? -Gv : Gv;
-          const double* eps = alpha ? s.ea : s.eb;
-          const double hdq = hdiag + eps[a] + eps[b] - eps[i] - eps[j] + G2at(I, i, j) + G2at(I, j, i) +
-                             G2at(I, a, b) + G2at(I, b, a) - G2at(I, a, i) - G2at(I, i, a) - G2at(I, b, i) -
-                             G2at(I, i, b) - G2at(I, a, j) - G2at(I, j, a) - G2at(I, b, j) - G2at(I, j, b);
-          if (alpha)
-            qa = ex;
-          else
-            qb = ex;
-          ch = c * h;
-          hd = A.E0 - hdq;
-          ok = true;
-        }
-      } else {
-        // append_os_doubles_asci_contributions (determinant_contributions.hpp:226-297)
-        x -= nda + ndb;
-        const int64_t xa = x / nsb, xb = x % nsb;
-        const uint32_t i = s.oa[xa / na_v], a = s.va[xa % na_v];
-        const uint32_t j = s.ob[xb / nb_v], b = s.vb[xb % nb_v];
-        const double V = Vat(I, a, i, b, j);
-        if (fabs(c * V) >= A.h_el_tol) {
-          const double sg = sgn(Pa, a, i) * sgn(Pb, b, j);
-          const double hdq = hdiag + s.ea[a] + s.eb[b] - s.ea[i] - s.eb[j] + V2at(I, i, j) + V2at(I, a, b) -
-                             G2at(I, a, i) - G2at(I, i, a) - G2at(I, b, j) - G2at(I, j, b) - V2at(I, a, j) -
-                             V2at(I, i, b);
-          qa = (Pa ^ (1ull << i)) | (1ull << a);
-          qb = (Pb ^ (1ull << j)) | (1ull << b);
-          ch = c * sg * V;
-          hd = A.E0 - hdq;
-          ok = true;
-        }
-      }
-      if (ok && (A.npass == 1 || part_of(qa, qb, A.npass) == A.pass)) table_add(A.T, qa, qb, ch, hd);
-    }
-    __syncwarp();
-    (void)full;
-  }
-}
-
 // Number of distinct target determinants of an enumeration (every single
 // and double of every core determinant, and the core itself) as a
 // HyperLogLog sketch: 2^kHllBits registers hold the largest leading-zero rank
@@ -314,99 +193,394 @@ __device__ __forceinline__ void hll_add(unsigned* reg, uint64_t qa, uint64_t qb)
   const unsigned rank = w ? (unsigned)__clzll(w) + 1u : (unsigned)(64 - kHllBits + 1);
   if (reg[idx] < rank) atomicMax(reg + idx, rank);
 }
-__global__ void __launch_bounds__(kAsciWarps * 32) k_target_sketch(CoreArgs A, unsigned* __restrict__ regs) {
-  __shared__ unsigned sreg[kHllRegs];
-  __shared__ WarpSm wsm[kAsciWarps];
-  for (int i = threadIdx.x; i < kHllRegs; i += blockDim.x) sreg[i] = 0u;
-  __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  WarpSm& s = wsm[w];
-  const int n = A.n;
-  for (int64_t ip = (int64_t)blockIdx.x * kAsciWarps + w; ip < A.ncore; ip += (int64_t)gridDim.x * kAsciWarps) {
-    const uint64_t Pa = A.ca[ip], Pb = A.cb[ip];
-    const int ka = popc64(Pa), kb = popc64(Pb), na_v = n - ka, nb_v = n - kb;
-    if (lane == 0) {
-      int x = 0, y = 0, u = 0, v = 0;
-      for (int p = 0; p < n; ++p) {
-        if ((Pa >> p) & 1)
-          s.oa[x++] = p;
-        else
-          s.va[y++] = p;
-        if ((Pb >> p) & 1)
-          s.ob[u++] = p;
-        else
-          s.vb[v++] = p;
-      }
-      hll_add(sreg, Pa, Pb);
-    }
-    __syncwarp();
-    const int64_t nsa = (int64_t)ka * na_v, nsb = (int64_t)kb * nb_v;
-    const int64_t pa_v = (int64_t)na_v * (na_v - 1) / 2, pb_v = (int64_t)nb_v * (nb_v - 1) / 2;
-    const int64_t nda = (int64_t)ka * (ka - 1) / 2 * pa_v, ndb = (int64_t)kb * (kb - 1) / 2 * pb_v;
-    const int64_t total = A.just_singles ? nsa + nsb : nsa + nsb + nda + ndb + nsa * nsb;
-    for (int64_t e = lane; e < total; e += 32) {
-      uint64_t qa = Pa, qb = Pb;
-      int64_t x = e;
-      if (x < nsa + nsb) {
-        const bool alpha = x < nsa;
-        if (!alpha) x -= nsa;
-        const int nv = alpha ? na_v : nb_v;
-        const uint32_t i = alpha ? s.oa[x / nv] : s.ob[x / nv];
-        const uint32_t a = alpha ? s.va[x % nv] : s.vb[x % nv];
-        if (alpha)
-          qa = (Pa ^ (1ull << i)) | (1ull << a);
-        else
-          qb = (Pb ^ (1ull << i)) | (1ull << a);
-      } else if ((x -= nsa + nsb) < nda + ndb) {
-        const bool alpha = x < nda;
-        if (!alpha) x -= nda;
-        const int64_t pv = alpha ? pa_v : pb_v;
-        int ii, jj, aa, bb;
-        pair_of((int)(x / pv), ii, jj);
-        pair_of((int)(x % pv), aa, bb);
-        const uint8_t* occ = alpha ? s.oa : s.ob;
-        const uint8_t* vir = alpha ? s.va : s.vb;
-        const uint64_t full = (1ull << occ[ii]) | (1ull << occ[jj]) | (1ull << vir[aa]) | (1ull << vir[bb]);
-        if (alpha)
-          qa = Pa ^ full;
-        else
-          qb = Pb ^ full;
-      } else {
-        x -= nda + ndb;
-        const int64_t xa = x / nsb, xb = x % nsb;
-        qa = (Pa ^ (1ull << s.oa[xa / na_v])) | (1ull << s.va[xa % na_v]);
-        qb = (Pb ^ (1ull << s.ob[xb / nb_v])) | (1ull << s.vb[xb % nb_v]);
-      }
-      hll_add(sreg, qa, qb);
-    }
-    __syncwarp();
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < kHllRegs; i += blockDim.x)
-    if (sreg[i]) atomicMax(regs + i, sreg[i]);
+
+// What a CTA holds of its core determinant, sized by the determinant's own
+// counts: singles as (occupied, virtual, sign) and their two G2 elements,
+// pairs of occupied and of virtual orbitals.  At most 46 KB (64 orbitals,
+// half of them occupied).
+__host__ __device__ inline size_t asci_smem(bool count, int n, int ka, int kb, bool just_singles) {
+  const size_t ns = (size_t)ka * (n - ka) + (size_t)kb * (n - kb);
+  const size_t np = just_singles ? 0
+                                 : ((size_t)ka * (ka - 1) + (size_t)(n - ka) * (n - ka - 1) + (size_t)kb * (kb - 1) +
+                                    (size_t)(n - kb) * (n - kb - 1)) /
+                                       2;
+  const size_t terms = (size_t)ka + kb + (size_t)ka * ka + (size_t)kb * kb + (size_t)ka * kb;
+  const size_t head = count ? kHllRegs * sizeof(unsigned) : (ns * 16 > terms * 8 ? ns * 16 : (terms * 8 + 15) / 16 * 16);
+  return head + 2 * (ns + np) + 16;
 }
 
-// candidates: finite score with |rv| > prune; key = bit pattern of |rv|
-__global__ void k_asci_extract(Table T, uint64_t cap, double prune, uint64_t* __restrict__ keys,
-                               uint64_t* __restrict__ slots, unsigned long long* __restrict__ count) {
+// Singles and doubles of every core determinant: inserted with their
+// contributions and diagonals (COUNT: into the sketch `regs`).  nslice CTAs
+// per determinant, a warp per row, lanes along the row: an alpha-beta row is
+// one beta single against every alpha single (integrals contiguous in the
+// lanes' index, the row's share of the diagonal loaded once), a same-spin row
+// one pair of occupied orbitals against every pair of virtual ones.  A warp
+// per determinant left most of the chip idle at the usual few thousand core
+// determinants, and spent 64-bit divisions on every target.  The order of the
+// FP64 operations of each contribution and diagonal is the reference's.
+//
+// Four searches from up to 1,000 of 8+8 electrons in 40 orbitals (141 million
+// contributions above the threshold in the largest): 62.8 -> 17.6 ms, the
+// sketch 6.3 -> 0.6.  What bounds it: the FP64 pipe for 60% of the time (23
+// instructions a contribution, of which 14 are the diagonal, whose rounding
+// the selection between spin-flipped twins depends on), and the round trips
+// to a table that no cache holds.  Looking at the slot before the exchange
+// cost more than the exchanges it saved.
+template <bool COUNT>
+__global__ void __launch_bounds__(kAsciWarps * 32, 4) k_asci_enum(CoreArgs A, unsigned* __restrict__ regs) {
+  extern __shared__ __align__(16) unsigned char dyn[];
+  __shared__ double ea[kMaxOrb], eb[kMaxOrb], hdiag_s;
+  __shared__ uint8_t oa[kMaxOrb], va[kMaxOrb], ob[kMaxOrb], vb[kMaxOrb];
+  __shared__ double pend_ch[COUNT ? 1 : kAsciWarps][64];
+  __shared__ uint16_t pend_x[COUNT ? 1 : kAsciWarps][64];
+  constexpr int kThreads = kAsciWarps * 32;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const Integrals& I = A.I;
+  const int n = A.n;
+  const size_t nn = (size_t)n;
+  const int64_t ip = blockIdx.x / A.nslice;
+  const int slice = (int)(blockIdx.x % A.nslice);
+  const uint64_t Pa = A.ca[ip], Pb = A.cb[ip];
+  const double c = A.cc[ip];
+  const int ka = popc64(Pa), kb = popc64(Pb), na_v = n - ka, nb_v = n - kb;
+  const int nsa = ka * na_v, nsb = kb * nb_v;
+  const int pa_o = ka * (ka - 1) / 2, pb_o = kb * (kb - 1) / 2;
+  const int pa_v = na_v * (na_v - 1) / 2, pb_v = nb_v * (nb_v - 1) / 2;
+  const int terms = ka + kb + ka * ka + kb * kb + ka * kb;
+  double2* sg = reinterpret_cast<double2*>(dyn);  // (G2(a, i), G2(i, a)) per single, beta's after alpha's
+  unsigned* hll = reinterpret_cast<unsigned*>(dyn);
+  const size_t head =
+      COUNT ? kHllRegs * sizeof(unsigned)
+            : (size_t)max(16 * (nsa + nsb), (terms * 8 + 15) / 16 * 16);
+  uint16_t* sgl = reinterpret_cast<uint16_t*>(dyn + head);  // i | a << 6 | sign << 12
+  uint16_t* pao = sgl + nsa + nsb;                          // i | j << 6, i < j
+  uint16_t *pav = pao + pa_o, *pbo = pav + pa_v, *pbv = pbo + pb_o;
+
+  if (tid < n) {
+    const uint64_t below = (1ull << tid) - 1ull;
+    const int x = popc64(Pa & below), y = popc64(Pb & below);
+    if ((Pa >> tid) & 1)
+      oa[x] = tid;
+    else
+      va[tid - x] = tid;
+    if ((Pb >> tid) & 1)
+      ob[y] = tid;
+    else
+      vb[tid - y] = tid;
+  }
+  if (COUNT)
+    for (int i = tid; i < kHllRegs; i += kThreads) hll[i] = 0u;
+  __syncthreads();
+  // orbital energies (single_orbital_ens, fast_diagonals.ipp:30-50) and the
+  // terms of the diagonal element in me_diag's order
+  if (!COUNT) {
+    if (tid < 2 * kMaxOrb) {
+      const bool alpha = tid < kMaxOrb;
+      const int i = tid & (kMaxOrb - 1);
+      const uint8_t *same = alpha ? oa : ob, *other = alpha ? ob : oa;
+      const int ks = alpha ? ka : kb, ko = alpha ? kb : ka;
+      if (i < n) {
+        double e = ld(I.T + i + nn * i);
+#pragma unroll 4
+        for (int x = 0; x < ks; ++x) {
+          const uint32_t q = same[x];
+          e += G2at(I, i, q) + G2at(I, q, i);
+        }
+        e -= G2at(I, i, i);
+#pragma unroll 4
+        for (int x = 0; x < ko; ++x) e += V2at(I, i, other[x]);
+        (alpha ? ea : eb)[i] = e;
+      }
+    } else {
+      double* term = reinterpret_cast<double*>(dyn);
+      for (int t = tid - 2 * kMaxOrb; t < terms; t += kThreads - 2 * kMaxOrb) {
+        int x = t;
+        const double* src;
+        if (x < ka)
+          src = I.T + oa[x] + nn * oa[x];
+        else if ((x -= ka) < kb)
+          src = I.T + ob[x] + nn * ob[x];
+        else if ((x -= kb) < ka * ka)
+          src = I.G2 + nn * oa[x / ka] + oa[x % ka];
+        else if ((x -= ka * ka) < kb * kb)
+          src = I.G2 + nn * ob[x / kb] + ob[x % kb];
+        else {
+          x -= kb * kb;
+          src = I.V2 + nn * ob[x / ka] + oa[x % ka];
+        }
+        term[t] = ld(src);
+      }
+    }
+  }
+  // singles and pairs
+  for (int x = tid; x < nsa + nsb; x += kThreads) {
+    const bool alpha = x < nsa;
+    const int y = alpha ? x : x - nsa, nv = alpha ? na_v : nb_v;
+    const uint32_t i = (alpha ? oa : ob)[y / nv], a = (alpha ? va : vb)[y % nv];
+    sgl[x] = (uint16_t)(i | (a << 6) | (excitation_sign_odd(alpha ? Pa : Pb, a, i) ? 1u << 12 : 0u));
+  }
+  if (!A.just_singles) {
+    // pairs (x, y), x < y: y runs fastest, rows x of K - 1 - x entries
+    auto pairs = [&](uint16_t* out, const uint8_t* list, int K) {
+      for (int t = tid; t < K * K; t += kThreads) {
+        const int x = t / K, y = t % K;
+        if (y > x) out[x * (2 * K - x - 1) / 2 + y - x - 1] = (uint16_t)(list[x] | (list[y] << 6));
+      }
+    };
+    pairs(pao, oa, ka);
+    pairs(pav, va, na_v);
+    pairs(pbo, ob, kb);
+    pairs(pbv, vb, nb_v);
+  }
+  __syncthreads();
+  if (!COUNT) {
+    if (tid == 0) {
+      const double* term = reinterpret_cast<const double*>(dyn);
+      double h = 0.;
+#pragma unroll 8
+      for (int t = 0; t < terms; ++t) h += term[t];
+      hdiag_s = h;
+    }
+    __syncthreads();
+    for (int x = tid; x < nsa + nsb; x += kThreads) {
+      const uint32_t i = sgl[x] & 63, a = (sgl[x] >> 6) & 63;
+      sg[x] = make_double2(G2at(I, a, i), G2at(I, i, a));
+    }
+    __syncthreads();
+  }
+  const double hdiag = COUNT ? 0. : hdiag_s;
+
+  // the core determinant itself: marked, removed later
+  if (slice == 0 && tid == 0) {
+    if (COUNT)
+      hll_add(hll, Pa, Pb);
+    else if (A.npass == 1 || part_of(Pa, Pb, A.npass) == A.pass)
+      table_add_core(A.T, Pa, Pb);
+  }
+  auto add = [&](uint64_t qa, uint64_t qb, double ch, auto diag) {
+    if (A.npass == 1 || part_of(qa, qb, A.npass) == A.pass) table_add(A.T, qa, qb, ch, diag);
+  };
+  // A row's N contributions ch(x), those that the threshold keeps gathered
+  // until a warp full of them (or the row's end) goes on to full(x, ch).
+  auto gather = [&](int N, auto contribution, auto full) {
+    double* qc = pend_ch[COUNT ? 0 : tid >> 5];
+    uint16_t* qx = pend_x[COUNT ? 0 : tid >> 5];
+    int held = 0;
+    for (int x0 = 0; x0 < N; x0 += 32) {
+      const int x = x0 + lane;
+      const double ch = x < N ? contribution(x) : 0.;
+      const bool keep = x < N && A.keeps(ch);
+      const unsigned m = __ballot_sync(QDKGB_FULL_MASK, keep);
+      if (keep) {
+        const int p = held + __popc(m & ((1u << lane) - 1u));
+        qc[p] = ch;
+        qx[p] = (uint16_t)x;
+      }
+      held += __popc(m);
+      __syncwarp();
+      const bool last = x0 + 32 >= N;
+      while (held >= 32 || (last && held > 0)) {
+        if (lane < held) full((int)qx[lane], qc[lane]);
+        __syncwarp();
+        held -= 32;
+        if (lane < held) {
+          qc[lane] = qc[32 + lane];
+          qx[lane] = qx[32 + lane];
+        }
+        __syncwarp();
+      }
+      held = max(held, 0);
+    }
+  };
+  const int r_os = A.just_singles || nsa == 0 ? 0 : nsb;
+  const int r_aa = A.just_singles ? 0 : pa_o, r_bb = A.just_singles ? 0 : pb_o;
+  const int nrows = r_os + r_aa + r_bb + 2;
+  for (int r = slice * kAsciWarps + (tid >> 5); r < nrows; r += A.nslice * kAsciWarps) {
+    if (r < r_os) {
+      // append_os_doubles_asci_contributions (determinant_contributions.hpp:226-297)
+      const uint32_t sb = sgl[nsa + r], j = sb & 63, b = (sb >> 6) & 63;
+      const uint64_t qb = (Pb ^ (1ull << j)) | (1ull << b);
+      const double* Vb = I.V + nn * nn * (b + nn * j);
+      double ebb, ebj, gbj, gjb;
+      if (!COUNT) ebb = eb[b], ebj = eb[j], gbj = sg[nsa + r].x, gjb = sg[nsa + r].y;
+      if (COUNT) {
+        for (int x = lane; x < nsa; x += 32) {
+          const uint32_t sa = sgl[x];
+          hll_add(hll, (Pa ^ (1ull << (sa & 63))) | (1ull << ((sa >> 6) & 63)), qb);
+        }
+        continue;
+      }
+      gather(
+          nsa,
+          [&](int x) {
+            const uint32_t sa = sgl[x];
+            return c * ld(Vb + ((sa >> 6) & 63) + nn * (sa & 63));
+          },
+          [&](int x, double ch) {
+            const uint32_t sa = sgl[x], i = sa & 63, a = (sa >> 6) & 63;
+            add((Pa ^ (1ull << i)) | (1ull << a), qb, ((sa ^ sb) >> 12) & 1 ? -ch : ch, [&] {
+              const double hdq = hdiag + ea[a] + ebb - ea[i] - ebj + V2at(I, i, j) + V2at(I, a, b) - sg[x].x -
+                                 sg[x].y - gbj - gjb - V2at(I, a, j) - V2at(I, i, b);
+              return A.E0 - hdq;
+            });
+          });
+    } else if (r < r_os + r_aa + r_bb) {
+      // append_ss_doubles_asci_contributions (determinant_contributions.hpp:149-210)
+      const bool alpha = r < r_os + r_aa;
+      const uint32_t po = alpha ? pao[r - r_os] : pbo[r - r_os - r_aa];
+      const uint16_t* pv = alpha ? pav : pbv;
+      const int npv = alpha ? pa_v : pb_v;
+      const uint32_t i = po & 63, j = po >> 6;
+      const uint64_t same = alpha ? Pa : Pb;
+      const double* eps = alpha ? ea : eb;
+      const uint64_t ij = (1ull << i) | (1ull << j);
+      if (COUNT) {
+        for (int x = lane; x < npv; x += 32) {
+          const uint64_t ex = same ^ (ij | (1ull << (pv[x] & 63)) | (1ull << (pv[x] >> 6)));
+          hll_add(hll, alpha ? ex : Pa, alpha ? Pb : ex);
+        }
+        continue;
+      }
+      gather(
+          npv,
+          [&](int x) {
+            const uint32_t a = pv[x] & 63, b = pv[x] >> 6;
+            return c * (Vat(I, b, j, a, i) - Vat(I, b, i, a, j));
+          },
+          [&](int x, double ch) {
+            const uint32_t a = pv[x] & 63, b = pv[x] >> 6;
+            const uint64_t fullex = ij | (1ull << a) | (1ull << b);
+            const uint64_t ex = same ^ fullex;
+            // doubles_sign(state_same, ex_det, full_ex): bra = P, ket = Q
+            SingleEx s1 = single_ex(same, ex, fullex);
+            const uint64_t f1 = (1ull << s1.o) | (1ull << s1.v);
+            SingleEx s2 = single_ex(same, ex ^ f1, fullex ^ f1);
+            add(alpha ? ex : Pa, alpha ? Pb : ex, s1.neg != s2.neg ? -ch : ch, [&] {
+              const double hdq = hdiag + eps[a] + eps[b] - eps[i] - eps[j] + G2at(I, i, j) + G2at(I, j, i) +
+                                 G2at(I, a, b) + G2at(I, b, a) - G2at(I, a, i) - G2at(I, i, a) - G2at(I, b, i) -
+                                 G2at(I, i, b) - G2at(I, a, j) - G2at(I, j, a) - G2at(I, b, j) - G2at(I, j, b);
+              return A.E0 - hdq;
+            });
+          });
+    } else {
+      // append_singles_asci_contributions (determinant_contributions.hpp:93-133)
+      const bool alpha = r == r_os + r_aa + r_bb;
+      const int x0 = alpha ? 0 : nsa, ns = alpha ? nsa : nsb;
+      const uint64_t same = alpha ? Pa : Pb, other = alpha ? Pb : Pa;
+      const double* eps = alpha ? ea : eb;
+      for (int x = lane; x < ns; x += 32) {
+        const uint32_t s1 = sgl[x0 + x], i = s1 & 63, a = (s1 >> 6) & 63;
+        const uint64_t ex = (same ^ (1ull << i)) | (1ull << a);
+        const uint64_t qa = alpha ? ex : Pa, qb = alpha ? Pb : ex;
+        if (COUNT) {
+          hll_add(hll, qa, qb);
+          continue;
+        }
+        double h = ld(I.T + a + nn * i);
+        const double* G = I.G_red + nn * (a + nn * i);
+        const double* Vr = I.V_red + nn * (a + nn * i);
+        for (uint64_t m = same; m; m &= m - 1) h += ld(G + low_bit(m));
+        for (uint64_t m = other; m; m &= m - 1) h += ld(Vr + low_bit(m));
+        if (A.keeps(c * h)) {
+          if ((s1 >> 12) & 1) h = -h;
+          add(qa, qb, c * h, [&] {
+            const double hdq = hdiag + eps[a] - eps[i] - sg[x0 + x].x - sg[x0 + x].y;
+            return A.E0 - hdq;
+          });
+        }
+      }
+    }
+  }
+  if (COUNT) {
+    __syncthreads();
+    for (int i = tid; i < kHllRegs; i += kThreads)
+      if (hll[i] > __ldcg(regs + i)) atomicMax(regs + i, hll[i]);
+  }
+}
+
+// The enumeration's launch shape: enough CTAs per core determinant to fill
+// the chip several times over (a determinant's tables are made by each of its
+// CTAs, so no more than that), and the shared memory of the largest one.
+struct EnumShape {
+  unsigned grid;
+  size_t smem_count, smem;
+};
+EnumShape enum_shape(const Context* c, CoreArgs& A, const uint64_t* ca, const uint64_t* cb) {
+  EnumShape e{0, 0, 0};
+  int rows = 1;
+  for (int64_t i = 0; i < A.ncore; ++i) {
+    const int ka = __builtin_popcountll(ca[i]), kb = __builtin_popcountll(cb[i]);
+    e.smem_count = std::max(e.smem_count, asci_smem(true, A.n, ka, kb, A.just_singles));
+    e.smem = std::max(e.smem, asci_smem(false, A.n, ka, kb, A.just_singles));
+    rows = std::max(rows, A.just_singles ? 2 : kb * (A.n - kb) + ka * (ka - 1) / 2 + kb * (kb - 1) / 2 + 2);
+  }
+  const int64_t fill = ((int64_t)c->sm_count * 32 + A.ncore - 1) / A.ncore;
+  A.nslice = (int)std::max<int64_t>(1, std::min<int64_t>(fill, (rows + kAsciWarps - 1) / kAsciWarps));
+  if (A.ncore * A.nslice > 0x7fffffff) throw Error(QDKGB_ERR_UNSUPPORTED, "ASCI: more than 2^31 core determinants");
+  e.grid = (unsigned)(A.ncore * A.nslice);
+  return e;
+}
+
+// candidates: finite score with |rv| > prune; key = bit pattern of |rv|.  A
+// CTA gathers the filled slots of a stretch in shared memory (half the table
+// is empty) and then divides with all lanes busy; one addition to the global
+// count per stretch (one per warp was a queue at that counter: 1.4 ms a search
+// over up to 130 million slots, 0.83 so).
+constexpr int kExtractSlots = 2048;
+__global__ void __launch_bounds__(256) k_asci_extract(Table T, uint64_t cap, double prune, uint64_t* __restrict__ keys,
+                                                      uint64_t* __restrict__ slots,
+                                                      unsigned long long* __restrict__ count) {
+  __shared__ uint16_t list[kExtractSlots];
+  __shared__ uint64_t skey[kExtractSlots];
+  __shared__ unsigned nlist, nkeep;
+  __shared__ unsigned long long base;
   const int lane = threadIdx.x & 31;
-  for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < cap; i0 += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t i = i0 + threadIdx.x;
-    bool take = false;
-    double arv = 0.;
-    if (i < cap && T.keys[i] != kEmpty && !table_core(T, i)) {
-      arv = fabs(table_sum(T, i) / __longlong_as_double(T.hd[i]));
-      take = arv > prune;
+  const unsigned below = (1u << lane) - 1u;
+  for (uint64_t i0 = (uint64_t)blockIdx.x * kExtractSlots; i0 < cap; i0 += (uint64_t)gridDim.x * kExtractSlots) {
+    if (threadIdx.x == 0) nlist = nkeep = 0;
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < kExtractSlots / 256; ++t) {
+      const unsigned x = t * 256 + threadIdx.x;
+      const bool full = i0 + x < cap && T.slot[i0 + x].key != kEmpty && !table_core(T, i0 + x);
+      const unsigned m = __ballot_sync(QDKGB_FULL_MASK, full);
+      unsigned p = 0;
+      if (lane == 0 && m) p = atomicAdd(&nlist, (unsigned)__popc(m));
+      p = __shfl_sync(QDKGB_FULL_MASK, p, 0);
+      if (full) list[p + __popc(m & below)] = (uint16_t)x;
     }
-    const unsigned m = __ballot_sync(QDKGB_FULL_MASK, take);
-    unsigned long long base = 0;
-    if (lane == 0 && m) base = atomicAdd(count, (unsigned long long)__popc(m));
-    base = __shfl_sync(QDKGB_FULL_MASK, base, 0);
-    if (take) {
-      const unsigned long long p = base + __popc(m & ((1u << lane) - 1u));
-      keys[p] = (uint64_t)__double_as_longlong(arv);
-      slots[p] = i;
+    __syncthreads();
+    const unsigned nl = nlist;
+    unsigned mine[kExtractSlots / 256];  // position among the kept ones
+#pragma unroll
+    for (int t = 0; t < kExtractSlots / 256; ++t) {
+      const unsigned y = t * 256 + threadIdx.x;
+      mine[t] = ~0u;
+      if (t * 256 >= nl) continue;
+      bool take = false;
+      double arv = 0.;
+      if (y < nl) {
+        arv = fabs(table_sum(T, i0 + list[y]) / __longlong_as_double(T.hd[i0 + list[y]]));
+        take = arv > prune;
+        skey[y] = (uint64_t)__double_as_longlong(arv);
+      }
+      const unsigned m = __ballot_sync(QDKGB_FULL_MASK, take);
+      unsigned p = 0;
+      if (lane == 0 && m) p = atomicAdd(&nkeep, (unsigned)__popc(m));
+      p = __shfl_sync(QDKGB_FULL_MASK, p, 0);
+      if (take) mine[t] = p + __popc(m & below);
     }
+    __syncthreads();
+    if (threadIdx.x == 0) base = nkeep ? atomicAdd(count, (unsigned long long)nkeep) : 0ull;
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < kExtractSlots / 256; ++t) {
+      const unsigned y = t * 256 + threadIdx.x;
+      if (mine[t] == ~0u) continue;
+      keys[base + mine[t]] = skey[y];
+      slots[base + mine[t]] = i0 + list[y];
+    }
+    __syncthreads();
   }
 }
 
@@ -442,7 +616,7 @@ __global__ void k_asci_select(const uint64_t* __restrict__ keys, const uint64_t*
     base = __shfl_sync(QDKGB_FULL_MASK, base, 0);
     if (take) {
       const unsigned long long p = base + __popc(m & ((1u << lane) - 1u));
-      const u128 key = T.keys[slots[i]];
+      const u128 key = T.slot[slots[i]].key;
       oa[p] = (uint64_t)key;
       ob[p] = (uint64_t)(key >> 64);
     }
@@ -458,7 +632,7 @@ __global__ void __launch_bounds__(256) k_pt2_sum(Table T, uint64_t cap, double* 
   double s = 0.;
   unsigned long long m = 0;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += (uint64_t)gridDim.x * blockDim.x) {
-    if (T.keys[i] != kEmpty && !table_core(T, i)) {
+    if (T.slot[i].key != kEmpty && !table_core(T, i)) {
       const double v = table_sum(T, i);
       s += v * v / __longlong_as_double(T.hd[i]);
       ++m;
@@ -485,9 +659,7 @@ __global__ void __launch_bounds__(256) k_pt2_sum(Table T, uint64_t cap, double* 
 
 __global__ void k_fill_empty(Table T, uint64_t cap) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += (uint64_t)gridDim.x * blockDim.x) {
-    T.keys[i] = kEmpty;
-    T.acc[2 * i] = 0;
-    T.acc[2 * i + 1] = 0;
+    T.slot[i] = Slot{kEmpty, 0, 0};
     T.hd[i] = kHdEmpty;
   }
 }
@@ -499,13 +671,18 @@ int64_t binom64(int n, int k) {
   return (int64_t)std::llround(r);
 }
 
+// Slots per estimated distinct target: the table is at most half full, two to
+// three probes (in one or two 128-byte lines) for a new target.  Rounded up
+// to a power of two from 2.5, as it was, a search allocated, filled and read
+// up to 2.5 times as many.
+constexpr double kSlotsPerTarget = 2.;
+
 // HyperLogLog estimate of the distinct targets of an enumeration over the
 // core list already on the device in A (small-range correction by linear
 // counting); `regs` is kHllRegs device words of scratch
-double distinct_targets(Context* c, const CoreArgs& A, unsigned* regs) {
+double distinct_targets(Context* c, const CoreArgs& A, const EnumShape& es, unsigned* regs) {
   QDKGB_CUDA(cudaMemsetAsync(regs, 0, kHllRegs * sizeof(unsigned), c->stream));
-  const unsigned eb = (unsigned)std::min<int64_t>((A.ncore + kAsciWarps - 1) / kAsciWarps, (int64_t)c->sm_count * 8);
-  k_target_sketch<<<eb, kAsciWarps * 32, 0, c->stream>>>(A, regs);
+  k_asci_enum<true><<<es.grid, kAsciWarps * 32, es.smem_count, c->stream>>>(A, regs);
   QDKGB_CHECK_LAUNCH();
   std::vector<unsigned> h(kHllRegs);
   QDKGB_CUDA(cudaMemcpyAsync(h.data(), regs, kHllRegs * sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
@@ -544,10 +721,10 @@ void asci_search_gpu(Context* c, int64_t ncore, const uint64_t* ca, const uint64
     const int64_t sa = (int64_t)ka * (n - ka), sb = (int64_t)kb * (n - kb);
     total += sa + sb + sa * sb + binom64(ka, 2) * binom64(n - ka, 2) + binom64(kb, 2) * binom64(n - kb, 2);
   }
-  ScopedBuffers<11> scratch(c);
-  DeviceBuffer &bkeys = scratch.b[0], &bsum = scratch.b[1], &bhd = scratch.b[2], &bck = scratch.b[3],
+  ScopedBuffers<10> scratch(c);
+  DeviceBuffer &bslot = scratch.b[0], &bhll = scratch.b[1], &bhd = scratch.b[2], &bck = scratch.b[3],
                &bcs = scratch.b[4], &bcnt = scratch.b[5], &berr = scratch.b[6], &bcore = scratch.b[7],
-               &bout = scratch.b[8], &bhist = scratch.b[9], &bhll = scratch.b[10];
+               &bout = scratch.b[8], &bhist = scratch.b[9];
   uint64_t* dcore = dev_array<uint64_t>(c, bcore, 3 * ncore);
   QDKGB_CUDA(cudaMemcpyAsync(dcore, ca, ncore * 8, cudaMemcpyHostToDevice, c->stream));
   QDKGB_CUDA(cudaMemcpyAsync(dcore + ncore, cb, ncore * 8, cudaMemcpyHostToDevice, c->stream));
@@ -565,26 +742,22 @@ void asci_search_gpu(Context* c, int64_t ncore, const uint64_t* ca, const uint64
   A.E0 = E0;
   A.h_el_tol = h_el_tol;
   A.just_singles = just_singles;
-  // table: 2.5 x the estimated distinct targets (at most 1.5 x the
+  // table: kSlotsPerTarget x the estimated distinct targets (at most 1.5 x the
   // contributions); an overflowing enumeration is redone with twice the slots
-  const double est = distinct_targets(c, A, dev_array<unsigned>(c, bhll, kHllRegs));
-  const double want = std::min((double)(total + total / 2), 2.5 * est + 2. * (double)ncore) + 1024.;
-  uint64_t cap = 1024;
-  while ((double)cap < want) cap <<= 1;
+  const EnumShape es = enum_shape(c, A, ca, cb);
+  const double est = distinct_targets(c, A, es, dev_array<unsigned>(c, bhll, kHllRegs));
+  uint64_t cap = (uint64_t)(std::min((double)(total + total / 2), kSlotsPerTarget * est + 2. * (double)ncore) + 1024.);
   size_t freeb = 0, totb = 0;
   QDKGB_CUDA(cudaMemGetInfo(&freeb, &totb));
   const size_t slot_bytes = 16 + 16 + 8 + 16;  // key, fixed-point sum, hd, candidate key + slot
   if (cap * slot_bytes > freeb / 2) throw Error(QDKGB_ERR_OOM, "ASCI search: hash table does not fit in device memory");
-  const unsigned eb = (unsigned)std::min<int64_t>((ncore + kAsciWarps - 1) / kAsciWarps, (int64_t)c->sm_count * 16);
   for (;;) {
-    u128* keys = (u128*)dev_alloc(c, bkeys, cap * 16 + 256);
-    keys = (u128*)(((uintptr_t)keys + 15) & ~(uintptr_t)15);
-    A.T = Table{keys, dev_array<long long>(c, bsum, 2 * cap), dev_array<long long>(c, bhd, cap), cap - 1, err};
+    A.T = Table{dev_array<Slot>(c, bslot, cap), dev_array<long long>(c, bhd, cap), cap, err};
     const unsigned fb = (unsigned)std::min<uint64_t>((cap + 255) / 256, (uint64_t)c->sm_count * 64);
     QDKGB_CUDA(cudaMemsetAsync(err, 0, sizeof(int), c->stream));
     k_fill_empty<<<fb, 256, 0, c->stream>>>(A.T, cap);
     QDKGB_CHECK_LAUNCH();
-    k_asci_enum<<<eb, kAsciWarps * 32, 0, c->stream>>>(A);
+    k_asci_enum<false><<<es.grid, kAsciWarps * 32, es.smem, c->stream>>>(A, nullptr);
     QDKGB_CHECK_LAUNCH();
     int herr = 0;
     QDKGB_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -597,7 +770,8 @@ void asci_search_gpu(Context* c, int64_t ncore, const uint64_t* ca, const uint64
   const unsigned fb = (unsigned)std::min<uint64_t>((cap + 255) / 256, (uint64_t)c->sm_count * 64);
   uint64_t* ckeys = dev_array<uint64_t>(c, bck, cap);
   uint64_t* cslots = dev_array<uint64_t>(c, bcs, cap);
-  k_asci_extract<<<fb, 256, 0, c->stream>>>(A.T, cap, rv_prune_tol, ckeys, cslots, cnt);
+  k_asci_extract<<<(unsigned)std::min<uint64_t>((cap + kExtractSlots - 1) / kExtractSlots, (uint64_t)c->sm_count * 32), 256, 0,
+                   c->stream>>>(A.T, cap, rv_prune_tol, ckeys, cslots, cnt);
   QDKGB_CHECK_LAUNCH();
   int herr = 0;
   unsigned long long ncand = 0;
@@ -693,9 +867,9 @@ double asci_pt2_gpu(Context* c, int64_t nd, const uint64_t* a, const uint64_t* b
     const int64_t sa = (int64_t)ka * (n - ka), sb = (int64_t)kb * (n - kb);
     total += sa + sb + sa * sb + binom64(ka, 2) * binom64(n - ka, 2) + binom64(kb, 2) * binom64(n - kb, 2);
   }
-  ScopedBuffers<7> scratch(c);
-  DeviceBuffer &bkeys = scratch.b[0], &bsum = scratch.b[1], &bhd = scratch.b[2], &berr = scratch.b[3],
-               &bcore = scratch.b[4], &bpart = scratch.b[5], &bhll = scratch.b[6];
+  ScopedBuffers<6> scratch(c);
+  DeviceBuffer &bslot = scratch.b[0], &bhll = scratch.b[1], &bhd = scratch.b[2], &berr = scratch.b[3],
+               &bcore = scratch.b[4], &bpart = scratch.b[5];
   uint64_t* dcore = dev_array<uint64_t>(c, bcore, 3 * nd);
   QDKGB_CUDA(cudaMemcpyAsync(dcore, a, nd * 8, cudaMemcpyHostToDevice, c->stream));
   QDKGB_CUDA(cudaMemcpyAsync(dcore + nd, b, nd * 8, cudaMemcpyHostToDevice, c->stream));
@@ -710,28 +884,28 @@ double asci_pt2_gpu(Context* c, int64_t nd, const uint64_t* a, const uint64_t* b
   A.cc = (const double*)(dcore + 2 * nd);
   A.E0 = E0;
   A.h_el_tol = pt2_tol;
-  // table: 2.5 x the estimated distinct targets (at most 1.5 x the
+  // table: kSlotsPerTarget x the estimated distinct targets (at most 1.5 x the
   // contributions), split into passes when it exceeds half the free memory or
   // max_slots; a pass whose probing overflows is redone with twice the slots
-  const double est = distinct_targets(c, A, dev_array<unsigned>(c, bhll, kHllRegs));
-  const double want = std::min((double)(total + total / 2), 2.5 * est + 2. * (double)nd) + 1024.;
-  uint64_t need = 1024;
-  while ((double)need < want) need <<= 1;
+  const EnumShape es = enum_shape(c, A, a, b);
+  const double est = distinct_targets(c, A, es, dev_array<unsigned>(c, bhll, kHllRegs));
+  const uint64_t need =
+      (uint64_t)(std::min((double)(total + total / 2), kSlotsPerTarget * est + 2. * (double)nd) + 1024.);
   size_t freeb = 0, totb = 0;
   QDKGB_CUDA(cudaMemGetInfo(&freeb, &totb));
   const size_t slot_bytes = 16 + 16 + 8;  // key, fixed-point sum, E0 - H_QQ
   const size_t budget = freeb / 2;
   const uint64_t slot_max = max_slots > 0 ? std::max<uint64_t>((uint64_t)max_slots, 1024) : ~0ull;
   auto fits = [&](uint64_t cp) { return cp * slot_bytes <= budget && cp <= slot_max; };
-  uint64_t cap = 1024;
-  while (cap < need && fits(cap << 1)) cap <<= 1;
+  uint64_t cap = need;
+  if (!fits(need))
+    for (cap = 1024; cap < need && fits(cap << 1);) cap <<= 1;
   const uint64_t npass = std::max<uint64_t>(1, (need + cap - 1) / cap);
   if (npass > 0xffffffffull) throw Error(QDKGB_ERR_OOM, "ASCI PT2: too many passes for the device memory");
   A.npass = (uint32_t)npass;
   const unsigned sb = (unsigned)std::min<uint64_t>((need + 255) / 256, (uint64_t)c->sm_count * 8);
   double* partial = (double*)dev_alloc(c, bpart, (size_t)sb * 16 + 64);
   unsigned long long* pcount = (unsigned long long*)(partial + sb);
-  const unsigned eb = (unsigned)std::min<int64_t>((nd + kAsciWarps - 1) / kAsciWarps, (int64_t)c->sm_count * 16);
   std::vector<double> hp(sb);
   std::vector<unsigned long long> hc(sb);
   double ept2 = 0.;
@@ -739,14 +913,12 @@ double asci_pt2_gpu(Context* c, int64_t nd, const uint64_t* a, const uint64_t* b
   for (uint64_t pass = 0; pass < npass; ++pass) {
     A.pass = (uint32_t)pass;
     for (;;) {
-      u128* keys = (u128*)dev_alloc(c, bkeys, cap * 16 + 256);
-      keys = (u128*)(((uintptr_t)keys + 15) & ~(uintptr_t)15);
-      A.T = Table{keys, dev_array<long long>(c, bsum, 2 * cap), dev_array<long long>(c, bhd, cap), cap - 1, err};
+      A.T = Table{dev_array<Slot>(c, bslot, cap), dev_array<long long>(c, bhd, cap), cap, err};
       const unsigned fb = (unsigned)std::min<uint64_t>((cap + 255) / 256, (uint64_t)c->sm_count * 64);
       QDKGB_CUDA(cudaMemsetAsync(err, 0, sizeof(int), c->stream));
       k_fill_empty<<<fb, 256, 0, c->stream>>>(A.T, cap);
       QDKGB_CHECK_LAUNCH();
-      k_asci_enum<<<eb, kAsciWarps * 32, 0, c->stream>>>(A);
+      k_asci_enum<false><<<es.grid, kAsciWarps * 32, es.smem, c->stream>>>(A, nullptr);
       QDKGB_CHECK_LAUNCH();
       k_pt2_sum<<<sb, 256, 0, c->stream>>>(A.T, cap, partial, pcount);
       QDKGB_CHECK_LAUNCH();
