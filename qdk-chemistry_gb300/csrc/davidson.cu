@@ -43,6 +43,16 @@ constexpr int kVecBlocksPerSm = 4;
 constexpr int kDotCols = 8;  // columns per block of k_multidot (one per warp in its final sum)
 constexpr int kDotChunks = (kMaxSubspace + 2 + kDotCols - 1) / kDotCols;
 
+// A load that stays where it is written: left to itself the compiler spreads
+// the sixteen loads of a step of k_df_ritz_residual between the arithmetic to
+// save registers (853,776 rows: 81.9 -> 73.1 us; the kernels with half as many
+// loads a step, and the FP64 ones, lose by it).
+__device__ __forceinline__ float2 ld_ahead(const float2* p) {
+  float2 v;
+  asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+
 // Sum of v over the block, valid in thread 0 (red: kVecThreads/32 doubles).
 __device__ __forceinline__ double block_sum_vec(double v, double* red) {
   v = warp_sum(v);
@@ -704,6 +714,7 @@ __global__ void __launch_bounds__(kVecThreads)
   for (int64_t i = (int64_t)blockIdx.x * kVecTile + threadIdx.x; i < n; i += step) {
     const int64_t i1 = i + kVecThreads;
     const bool has1 = i1 < n;
+    const int64_t in1 = has1 ? i1 : i;
     float2 x0 = zero, ax0 = zero, x1 = zero, ax1 = zero;
     int j = 0;
     for (; j + 4 <= k; j += 4) {
@@ -711,10 +722,10 @@ __global__ void __launch_bounds__(kVecThreads)
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const size_t o = (size_t)(j + q) * ld;
-        v0[q] = V[i + o];
-        w0[q] = AV[i + o];
-        v1[q] = has1 ? V[i1 + o] : zero;
-        w1[q] = has1 ? AV[i1 + o] : zero;
+        v0[q] = ld_ahead(V + i + o);
+        w0[q] = ld_ahead(AV + i + o);
+        v1[q] = ld_ahead(V + in1 + o);
+        w1[q] = ld_ahead(AV + in1 + o);
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
@@ -775,6 +786,27 @@ __global__ void k_df_from_f32(const float* __restrict__ x, float2* __restrict__ 
 __global__ void k_df_to_f64(const float2* __restrict__ x, double* __restrict__ y, int64_t n) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     y[i] = df::to_double(x[i]);
+}
+// |x - x^T|^2, |x + x^T|^2 and |x|^2 of an nstr x nstr vector, per block
+// (partial[3 b ...]): the spin-flip sector of a guess.  853,776 elements
+// 0.02 ms; copied to the host and added there, 4 ms of a 61 ms solve.
+__global__ void __launch_bounds__(256) k_flip_parity(const double* __restrict__ x, int64_t nstr,
+                                                     double* __restrict__ partial) {
+  __shared__ double red[kVecThreads / 32];
+  double dp = 0., dm = 0., nn = 0.;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < nstr * nstr; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = t / nstr, j = t - i * nstr;
+    const double a = x[t], b = x[j * nstr + i];
+    dp = fma(a - b, a - b, dp);
+    dm = fma(a + b, a + b, dm);
+    nn = fma(a, a, nn);
+  }
+  const double s[3] = {dp, dm, nn};
+  for (int q = 0; q < 3; ++q) {
+    const double v = block_sum_vec(s[q], red);
+    if (threadIdx.x == 0) partial[3 * blockIdx.x + q] = v;
+    __syncthreads();
+  }
 }
 // k_flip_project in double-float: x <- (x + s x^T) / 2 (s = +-1, so s x and
 // the halving are exact)
@@ -890,6 +922,7 @@ struct Dav {
   int nb;  // blocks of the row-parallel kernels (partial sums per column)
   int sm_count;
   double* gA = nullptr;
+  bool steady = false;  // every rounding as in the plain algorithm (ASCI)
   EigWarm* warm = nullptr;  // the projected problem's state from size to size
   cudaStream_t st;
 
@@ -898,12 +931,14 @@ struct Dav {
   double* col(double* base, int64_t j) { return base + (size_t)j * n; }
 
   // out[j * stride] = A[:, j] . w, j < k: column blocks of kDotCols on
-  // grid.y, the row split on grid.x shrunk as column blocks are added (down to
-  // one block per SM) so the grid stays near one resident wave
+  // grid.y, the row split on grid.x shrunk as column blocks are added so that
+  // the grid is one resident wave (854 thousand rows, 55 columns: 128 -> 114
+  // us against at least one block per SM and column block, up to 1.75 waves;
+  // a steady solve keeps that split)
   void multidot(const double* A, int k, const double* w, double* out, int stride, double* self_out = nullptr,
                 const double* skip = nullptr, int hrow = -1) {
     const int chunks = (k + kDotCols - 1) / kDotCols;
-    const int bx = std::max(1, std::min(nb, std::max(sm_count, nb / chunks)));
+    const int bx = std::max(1, std::min(nb, steady ? std::max(sm_count, nb / chunks) : sm_count * kVecBlocksPerSm / chunks));
     k_multidot<<<dim3(bx, chunks), kVecThreads, 0, st>>>(A, n, k, w, n, partial, counts(), out, stride, self_out,
                                                          skip, hrow, hrow >= 0 ? Hk : nullptr, (int)(maxm + 1));
     QDKGB_CHECK_LAUNCH();
@@ -941,11 +976,30 @@ struct Dav {
   }
   void clear_flag() { QDKGB_CUDA(cudaMemsetAsync(small + kSlotFlag, 0, sizeof(double), st)); }
 
-  // Two CGS passes against V[:, 0:K] (the reference always makes two).
-  // |w|^2 of the result goes to small[kSlotNrm].
+  // CGS passes against V[:, 0:K]; |w|^2 of the result goes to
+  // small[kSlotNrm].  The reference always makes two.  The second only
+  // removes what rounding left of the first, at most 2 eps of the result
+  // where that kept half of |w|^2 (Daniel, Gragg, Kaufman and Stewart, Math.
+  // Comp. 30, 772 (1976)): there it is skipped, which in these solves is
+  // nearly every time (12e12o, 854 thousand determinants: 184 -> 157 ms, the
+  // basis once instead of twice through the FP64 pipe that bounds both
+  // kernels).  A steady solve makes both: its result is to be the
+  // reference's to the last bit that the selection depends on.
   void orth_passes(int K, double* w) {
     if (K <= 0) {
       norm2(w, small + kSlotNrm);
+      return;
+    }
+    if (!steady) {
+      double* nrm = small + kSlotNrm;
+      multidot(V, K, w, small, 1, small + kSlotW2);
+      k_gemv_rows<true, true><<<nb, kVecThreads, 0, st>>>(V, n, K, small, 1, w, n, nullptr, small + kSlotW2,
+                                                          small + kSlotSkip, partial, counts(), nrm);
+      QDKGB_CHECK_LAUNCH();
+      multidot(V, K, w, small, 1, nullptr, small + kSlotSkip);
+      k_gemv_rows<true, true><<<nb, kVecThreads, 0, st>>>(V, n, K, small, 1, w, n, small + kSlotSkip, nullptr, nullptr,
+                                                          partial, counts(), nrm);
+      QDKGB_CHECK_LAUNCH();
       return;
     }
     multidot(V, K, w, small, 1);
@@ -1032,7 +1086,7 @@ struct Dav {
     }();
     const int nbd = (int)std::max<int64_t>(1, std::min<int64_t>((n + kVecTile - 1) / kVecTile, (int64_t)sm_count * per_sm));
     const int chunks = (k + kDotCols - 1) / kDotCols;
-    const int bx = std::max(1, std::min(nbd, std::max(sm_count, nbd / chunks)));
+    const int bx = std::max(1, std::min(nbd, sm_count * per_sm / chunks));
     k_df_multidot<<<dim3(bx, chunks), kVecThreads, 0, st>>>(A, n, k, w, n, partial, counts(), out, stride, self_out,
                                                             skip, hrow, hrow >= 0 ? Hk : nullptr, (int)(maxm + 1));
     QDKGB_CHECK_LAUNCH();
@@ -1152,6 +1206,7 @@ static void davidson_roots(Context* c, const qdkgb_davidson_settings* s, double*
   d.maxm = max_m;
   d.st = c->stream;
   d.sm_count = std::max(1, c->sm_count);
+  d.steady = true;  // two Gram-Schmidt passes: a block's directions can be nearly parallel
   d.nb = (int)std::max<int64_t>(1, std::min<int64_t>((N + kVecTile - 1) / kVecTile, (int64_t)d.sm_count * kVecBlocksPerSm));
   d.V = dev_array<double>(c, W.V, (size_t)N * (max_m + 1));
   d.AV = dev_array<double>(c, W.AV, (size_t)N * (max_m + 1));
@@ -1295,6 +1350,7 @@ void davidson(Context* c, const qdkgb_davidson_settings* s, double* E, double* C
   d.maxm = max_m;
   d.st = c->stream;
   d.sm_count = std::max(1, c->sm_count);
+  d.steady = steady;
   d.nb = (int)std::max<int64_t>(1, std::min<int64_t>((N + kVecTile - 1) / kVecTile, (int64_t)d.sm_count * kVecBlocksPerSm));
   d.V = dev_array<double>(c, W.V, (size_t)N * (max_m + 1));
   d.AV = dev_array<double>(c, W.AV, (size_t)N * (max_m + 1));
@@ -1465,17 +1521,19 @@ void davidson(Context* c, const qdkgb_davidson_settings* s, double* E, double* C
       for (int64_t g = 0; g < S.ngroups && square; ++g) square = (S.h_gstart[g + 1] - S.h_gstart[g]) == S.nbeta;
       if (square) {
         nstr = S.nbeta;
-        std::vector<double> g0(N);
-        QDKGB_CUDA(cudaMemcpyAsync(g0.data(), V0, N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+        const int fb = (int)std::min<int64_t>(d.nb, (N + 255) / 256);
+        k_flip_parity<<<fb, 256, 0, c->stream>>>(V0, nstr, d.partial);
+        QDKGB_CHECK_LAUNCH();
+        std::vector<double> part((size_t)3 * fb);
+        QDKGB_CUDA(cudaMemcpyAsync(part.data(), d.partial, part.size() * sizeof(double), cudaMemcpyDeviceToHost,
+                                   c->stream));
         QDKGB_CUDA(cudaStreamSynchronize(c->stream));
         double dp = 0., dm = 0., nn = 0.;
-        for (int64_t i = 0; i < nstr; ++i)
-          for (int64_t j = 0; j < nstr; ++j) {
-            const double x = g0[i * nstr + j], y = g0[j * nstr + i];
-            dp += (x - y) * (x - y);
-            dm += (x + y) * (x + y);
-            nn += x * x;
-          }
+        for (int b = 0; b < fb; ++b) {
+          dp += part[3 * b];
+          dm += part[3 * b + 1];
+          nn += part[3 * b + 2];
+        }
         if (dp <= 1e-24 * nn)
           flip = 1.;
         else if (dm <= 1e-24 * nn)
