@@ -126,7 +126,6 @@ void build_struct(Context* c) {
   // (index of the own-group / alpha-single block in the row, -1 for an
   // alpha double)
   int rowlen = -1, c1 = -1, c2 = -1;
-  PlanHost plan_tmp[2];
   std::vector<PlanHost> cand_tmp[2];
   std::vector<uint32_t> gdesc;
   std::vector<int32_t> pblock;  // [G][rowlen]
@@ -256,11 +255,19 @@ void build_struct(Context* c) {
       }
     }
     if (best_S < 0) return;
-    // the occupancy model's choice first, then the other feasible counts of
-    // at least 4 segments (fewer leave most SMs idle for these row counts)
+    // The occupancy model's choice first, then the three smallest feasible
+    // counts of at least 4 segments (fewer leave most SMs idle for these row
+    // counts) and 10.  Timed over all counts up to 16, the best of these was
+    // within 3% of the best of all from 400 to 853,776 determinants, and the
+    // others' timing (32 of 52 sigmas at 10e10o) and tables cost a solve of 73
+    // sigmas more than any choice could give back: 42 -> 32 ms with both.
     std::vector<int> cands{best_S};
+    int small = 0;
     for (int S : feasible)
-      if (S != best_S && S >= std::min(4, best_S)) cands.push_back(S);
+      if (S >= std::min(4, best_S) && (small < 3 || S == 10)) {
+        ++small;
+        if (S != best_S) cands.push_back(S);
+      }
     for (int S : cands) {
       const int M = shapeM[S], R = shapeR[S];
       std::vector<int32_t> rec((size_t)G * S * R, 0), segh((size_t)G * S * M, -1);
@@ -308,7 +315,6 @@ void build_struct(Context* c) {
       ph.R = R;
       ph.rec = std::move(rec);
       ph.segh = std::move(segh);
-      if (S == best_S) plan_tmp[pl] = ph;
       cand_tmp[pl].push_back(std::move(ph));
     }
   }
@@ -333,11 +339,11 @@ void build_struct(Context* c) {
   up(F->blT, blT.data(), blT.size() * 4);
   up(F->gdesc, gdesc.data(), gdesc.size() * 4);
   for (int pl = 0; pl < 2; ++pl) {
-    F->plan[pl].S = plan_tmp[pl].S;
-    F->plan[pl].M = plan_tmp[pl].M;
-    F->plan[pl].R = plan_tmp[pl].R;
-    up(F->plan[pl].rec, plan_tmp[pl].rec.data(), plan_tmp[pl].rec.size() * 4);
-    up(F->plan[pl].segh, plan_tmp[pl].segh.data(), plan_tmp[pl].segh.size() * 4);
+    F->plan[pl].S = cand_tmp[pl].front().S;
+    F->plan[pl].M = cand_tmp[pl].front().M;
+    F->plan[pl].R = cand_tmp[pl].front().R;
+    up(F->plan[pl].rec, cand_tmp[pl].front().rec.data(), cand_tmp[pl].front().rec.size() * 4);
+    up(F->plan[pl].segh, cand_tmp[pl].front().segh.data(), cand_tmp[pl].front().segh.size() * 4);
     F->cand[pl] = std::move(cand_tmp[pl]);
     F->tuned[pl] = F->cand[pl].size() <= 1;
   }
