@@ -33,6 +33,8 @@
 // are a ring of 64-column slots, one per group in flight, so the products of
 // the next chunk run under the read-out and the walk of this one.
 #pragma once
+#include <algorithm>
+
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -110,6 +112,21 @@ __device__ __forceinline__ double scale2(double v, int e) {
   if (x == 0 || x == 0x7ff) return v;  // zero (denormals do not arise from whole numbers)
   if (x + e > 0 && x + e < 0x7ff) return __hiloint2double(h + (e << 20), __double2loint(v));
   return ldexp(v, e);
+}
+// q 2^e rounded to FP64, to even as (double)q is, by integer instructions: a
+// conversion from 64-bit integers is several FP64 ones, 16 clocks a warp each
+// (a tile of k_dense64 took 17 us for its 16,384).
+static __device__ __noinline__ double whole_scaled_far(int64_t q, int e) { return ldexp((double)q, e); }
+__device__ __forceinline__ double whole_scaled(int64_t q, int e) {
+  if (q == 0) return 0.;
+  const uint64_t u = q < 0 ? 0ull - (uint64_t)q : (uint64_t)q;
+  const int lz = __clzll((long long)u);
+  const uint64_t m = u << lz, rest = m & 0x7ff;
+  uint64_t b = (m >> 11) + (uint64_t)(rest > 0x400 || (rest == 0x400 && (m & 0x800)));  // 2^52 .. 2^53
+  const int x = 1085 - lz + e;  // the exponent field, less the one that b's bit 52 adds
+  if (x < 0 || x > 2044) return whole_scaled_far(q, e);
+  b += (uint64_t)x << 52;
+  return __longlong_as_double((long long)(b | (q < 0 ? 1ull << 63 : 0ull)));
 }
 // balanced digits of q, most significant first: q = sum_i d[i] 2^(W (S-1-i))
 template <int S, int W>
@@ -194,11 +211,40 @@ struct Args {
   const double* D;
   const T* C;
   T* sigma;
-  const int* act;            // instances in use (null: all)
   const int* bad;            // FP64: non-finite input, leave the work to the plain form
-  int64_t s_sA, s_W, s_V2, s_vec, s_parts;
   unsigned* fault;
+  // FP64: alpha strings from `full` on are split over `split` CTAs each, by
+  // chunks (row_plan); their sums meet in part_lo / part_hi [CTA][nb] and
+  // part_count [string][arrived, failed] (zero before and after)
+  int full, split;
+  uint64_t* part_lo;
+  int32_t* part_hi;
+  unsigned* part_count;
 };
+
+// How the na alpha strings of the FP64 form go over `slots` SMs: whole ones in
+// full waves, those of a last, partly filled wave in `split` pieces of their
+// chunks (the pieces' sums are whole numbers and add exactly).  A CTA's start
+// and end take as long as about three chunks (12 orbitals: 17 + 4 thousand
+// clocks beside 8 thousand a chunk).  924 strings on 152 SMs were seven waves,
+// the last with 12 CTAs: 486 -> 447 us.  The FP32 form, two CTAs to an SM, has
+// its last wave's SMs to itself and lost by it (139.1 -> 146.6 us a sigma).
+struct RowPlan {
+  int full, split;
+};
+inline RowPlan row_plan(int na, int nchunk, int slots) {
+  const int rem = na % slots;
+  RowPlan best{na, 1};
+  int least = 1 << 30;
+  for (int s = 1; rem > 0 && s <= nchunk; ++s) {
+    const int waves = (int)(((int64_t)rem * s + slots - 1) / slots), cost = waves * (3 + (nchunk + s - 1) / s);
+    if (cost < least) {
+      least = cost;
+      best = s > 1 ? RowPlan{na - rem, s} : RowPlan{na, 1};
+    }
+  }
+  return best;
+}
 
 template <typename T>
 struct Form;
@@ -245,24 +291,20 @@ __global__ void __launch_bounds__((Form<T>::EpiWarps + 1 + kLoadWarps) * 32, For
   constexpr bool kF64 = sizeof(T) == 8;
   constexpr int S = F::S, G = F::G, kEpi = F::EpiWarps * 32, kPad = 16 * KS;
   constexpr int kSl = (F::Tmem - S * KS * 8) / kCols < 7 ? (F::Tmem - S * KS * 8) / kCols : 7;
-  static_assert(kSl >= 2, "accumulator ring");
+  static_assert(kSl >= 2 && (!kF64 || kSl >= 4), "accumulator slots");
+  // FP64: group gi of a chunk goes to slot gi % kSl.  A wait that need not
+  // wait costs 90 clocks on an idle SM and 350 here, so there are few: the
+  // read-out waits once for the first kSl groups and once for the rest, the
+  // products wait for the read-out of each group whose slot is used again in
+  // the chunk (kRe of them), of the last group in slot 0, and of the last.
+  constexpr int kRe = kF64 ? (G > kSl ? G - kSl : 0) : 0;
+  constexpr int kFirst = kRe > 0 ? kSl : 0;  // the last group in slot 0
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(8) uint64_t full[2], empty[2], accfull[kSl], accempty[kSl], listfull, done;
+  __shared__ __align__(8) uint64_t full[2], empty[2], accfull[kSl], accempty[kSl], reuse[kF64 ? G : 1], listfull, done;
   __shared__ uint32_t tslot;
-  __shared__ int fail_, mexp[2];
+  __shared__ int fail_, last_, mexp[2];
   volatile int* fail = &fail_;
-  {
-    const int inst = blockIdx.y;
-    if (g.act && !g.act[inst]) return;
-    if (kF64 && g.bad && *g.bad) return;
-    g.a_sA += inst * g.s_sA;
-    g.a_W += inst * g.s_W;
-    g.V2 += inst * g.s_V2;
-    g.D += inst * g.s_vec;
-    g.C += inst * g.s_vec;
-    g.sigma += inst * g.s_vec;
-    g.Cs += inst * g.s_parts;
-  }
+  if (kF64 && g.bad && *g.bad) return;
   const Smem<T> L(kPad, g.R, g.nb, g.seg_bytes);
   typename F::E* E = (typename F::E*)(smem + L.off_e);
   T* facc = (T*)(smem + L.off_acc);                    // FP32: the sums
@@ -272,10 +314,14 @@ __global__ void __launch_bounds__((Form<T>::EpiWarps + 1 + kLoadWarps) * 32, For
   int32_t* Jrow = (int32_t*)(smem + L.off_j);
   int32_t* kvo = Jrow + kPad;
   int32_t* kexp = kvo + kPad;
-  const int64_t Ia = blockIdx.x;
+  const bool whole = !kF64 || (int)blockIdx.x < g.full;
+  const int piece = whole ? 0 : (int)(blockIdx.x - g.full);  // among the split strings' CTAs
+  const int64_t Ia = whole ? (int64_t)blockIdx.x : g.full + piece / g.split;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int K = g.nsa + 1, n = g.n;
-  const int nchunk = (g.nb + kCols - 1) / kCols;
+  const int chunks = (g.nb + kCols - 1) / kCols, mine = whole ? 0 : piece % g.split;
+  const int chunk0 = whole ? 0 : mine * chunks / g.split;
+  const int nchunk = whole ? chunks : (mine + 1) * chunks / g.split - chunk0;
   if (warp == 0) tc::tmem_alloc(&tslot, F::Tmem);
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
@@ -286,6 +332,7 @@ __global__ void __launch_bounds__((Form<T>::EpiWarps + 1 + kLoadWarps) * 32, For
       tc::mbar_init(&accfull[i], 1);
       tc::mbar_init(&accempty[i], F::EpiWarps);
     }
+    for (int i = 0; i < (kF64 ? G : 1); ++i) tc::mbar_init(&reuse[i], F::EpiWarps);
     tc::mbar_init(&listfull, 1);
     tc::mbar_init(&done, 1);
     tc::mbar_init_fence();
@@ -412,7 +459,7 @@ __global__ void __launch_bounds__((Form<T>::EpiWarps + 1 + kLoadWarps) * 32, For
       const int buf = c & 1;
       if (c >= 2 && !wait(&empty[buf], (uint32_t)((c / 2 - 1) & 1), fail)) break;
       const uint32_t dst = tc::smem_addr(smem + buf * L.b_bytes);
-      const uint16_t* src = g.Cs + c * kCols;
+      const uint16_t* src = g.Cs + (chunk0 + c) * kCols;
       // item i: 16 bytes at 16 i; part i / (8 kPad), K row i % 8 of block (i / 64) % (kPad / 8), strings 8 ((i / 8) % 8) ..
 #pragma unroll 4
       for (int i = lt; i < items; i += kLt) {
@@ -436,16 +483,24 @@ __global__ void __launch_bounds__((Form<T>::EpiWarps + 1 + kLoadWarps) * 32, For
     int slot = 0;
     uint32_t round = 0;
     bool ok = true;
+    auto all_wait = [&](uint64_t* b, uint32_t parity) {
+      if (ok) ok = __all_sync(0xffffffffu, wait(b, parity, fail));
+    };
     for (int c = 0; c < nchunk && ok; ++c) {
       const int buf = c & 1;
-      ok = __all_sync(0xffffffffu, wait(&full[buf], (uint32_t)((c / 2) & 1), fail));
-      if (!ok) break;
-      tc::fence_after();
+      all_wait(&full[buf], (uint32_t)((c / 2) & 1));
       // MN-major: 8 x 8 core matrices, 128 bytes between 8-string blocks, 1024 between 8-row blocks
       const uint64_t db = tc::desc(tc::smem_addr(smem + buf * L.b_bytes), 1024, 128);
 #pragma unroll
       for (int gi = 0; gi < G; ++gi) {
-        if (ok && round > 0) ok = __all_sync(0xffffffffu, wait(&accempty[slot], (round - 1) & 1, fail));
+        if constexpr (kF64) {
+          if (gi >= kSl) all_wait(&reuse[gi - kSl], (uint32_t)(c & 1));
+          if (c > 0 && gi == 0) all_wait(&reuse[kFirst], (uint32_t)((c - 1) & 1));
+          if (c > 0 && gi == 1 && kFirst != G - 1) all_wait(&reuse[G - 1], (uint32_t)((c - 1) & 1));
+          slot = gi % kSl;
+        } else {
+          if (round > 0) all_wait(&accempty[slot], (round - 1) & 1);
+        }
         if (ok) {
           tc::fence_after();
           if (elect_one()) {
@@ -459,12 +514,14 @@ __global__ void __launch_bounds__((Form<T>::EpiWarps + 1 + kLoadWarps) * 32, For
                 for (int ks = 0; ks < KS; ++ks)
                   mma_f16_ts(d, tmem + (uint32_t)(i * KS * 8 + 8 * ks), db + (uint64_t)((p - i) * kPad * 8 + 128 * ks),
                              idesc, (p == p0 && i == 0 && ks == 0) ? 0u : 1u);
-            tc::commit(&accfull[slot]);
+            if (!kF64) tc::commit(&accfull[slot]);
+            if (kF64 && gi == min(kSl, G) - 1) tc::commit(&accfull[0]);
+            if (kF64 && kRe > 0 && gi == G - 1) tc::commit(&accfull[1]);
             if (gi == G - 1) tc::commit(&empty[buf]);
           }
           __syncwarp();
         }
-        if (++slot == kSl) {
+        if (!kF64 && ++slot == kSl) {
           slot = 0;
           ++round;
         }
@@ -490,48 +547,71 @@ __global__ void __launch_bounds__((Form<T>::EpiWarps + 1 + kLoadWarps) * 32, For
     }
     // the walk lists of a chunk: one bulk copy (TMA), completing on listfull
     auto load_list = [&](int c) {
-      const int u0 = __ldg(g.seg + c), bytes = 2 * (__ldg(g.seg + c + 1) - u0);
+      const int u0 = __ldg(g.seg + chunk0 + c), bytes = 2 * (__ldg(g.seg + chunk0 + c + 1) - u0);
       tc::mbar_expect_tx(&listfull, (uint32_t)bytes);
       tc::bulk_g2s(smem + L.off_list, g.walk + u0, (uint32_t)bytes, &listfull);
     };
     if (tid == 0) load_list(0);
     for (int c = 0; c < nchunk; ++c) {
       typename F::E ev[kW];
-      float low[kF64 ? kW : 1];
-      constexpr int64_t kMagic = 0x4b400000;
-      (void)low;
+      if constexpr (kF64) {
+        static_assert(kW == 16, "one TMEM load per group");
+        float low[16];
+        constexpr int64_t kMagic = 0x4b400000;
+        // units of 2^-57: group gr weighs 2^(57 - 9 (gr + 2)).  Groups 6 and 5
+        // meet in FP32 (below one unit and 2^-6 of a sum); |group 0| <= 2^16 K
+        // <= 2^22 and that pair become integers by the 1.5 2^23 addition
+        // (their bits, kMagic taken off), the others by a conversion.
+        auto take = [&](int gi, const float* v) {
 #pragma unroll
-      for (int gi = 0; gi < G; ++gi) {
-        constexpr int kTop = G - 1;
-        const int gr = kTop - gi;
+          for (int j = 0; j < 16; ++j) {
+            const float x = v[j];
+            if (gi == 0) low[j] = x * 0x1p-15f;
+            if (gi == 1)
+              ev[j] = (int64_t)(uint64_t)__float_as_uint(fmaf(x, 0x1p-6f, low[j]) + 12582912.f) - kMagic;
+            if (gi == 2) ev[j] += (int64_t)__float2int_rn(x) * (1 << 3);
+            if (gi == 3) ev[j] += (int64_t)__float2int_rn(x) * (1 << 12);
+            if (gi == 4) ev[j] += (int64_t)__float2int_rn(x) * (1 << 21);
+            if (gi == 5) ev[j] += (int64_t)__float2int_rn(x) * (1 << 30);
+            if (gi == 6) ev[j] += (int64_t)(((uint64_t)__float_as_uint(x + 12582912.f) - kMagic) << 39);
+          }
+        };
+        auto freed = [&](int gi) {
+          if (gi < kRe || gi == kFirst || gi == G - 1) {
+            tc::fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&reuse[gi]);
+          }
+        };
+        if (ok) ok = __all_sync(0xffffffffu, wait(&accfull[0], (uint32_t)(c & 1), fail));
+        tc::fence_after();
+#pragma unroll
+        for (int gi = 0; gi < G; ++gi) {
+          if (kRe > 0 && gi == kSl) {
+            if (ok) ok = __all_sync(0xffffffffu, wait(&accfull[1], (uint32_t)(c & 1), fail));
+            tc::fence_after();
+          }
+          // two groups under one wait for TMEM, not across the second wait above
+          const int first = gi < kSl ? 0 : kSl, past = gi < kSl ? min(kSl, G) : G;
+          if ((gi - first) & 1) continue;
+          float v0[16], v1[16];
+          if (gi + 1 < past) {
+            tc::tmem_ld16x2(tl + (uint32_t)(gi % kSl * kCols), tl + (uint32_t)((gi + 1) % kSl * kCols), v0, v1);
+            freed(gi);
+            freed(gi + 1);
+            take(gi, v0);
+            take(gi + 1, v1);
+          } else {
+            tc::tmem_ld16(tl + (uint32_t)(gi % kSl * kCols), v0);
+            freed(gi);
+            take(gi, v0);
+          }
+        }
+      } else {
         if (ok) ok = __all_sync(0xffffffffu, wait(&accfull[slot], round & 1, fail));
         tc::fence_after();
 #pragma unroll
-        for (int h = 0; h < kW; h += 16) {
-          float v[16];
-          tc::tmem_ld16(tl + (uint32_t)(slot * kCols + h), v);
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            if constexpr (kF64) {
-              // units of 2^-57: group gr weighs 2^(57 - 9 (gr + 2)).  Groups
-              // 6 and 5 meet in FP32 (below one unit and 2^-6 of a sum);
-              // |group 0| <= 2^16 K <= 2^22 and that pair become integers by
-              // the 1.5 2^23 addition (their bits, kMagic taken off at the
-              // end), the others by a conversion: those run at 16 a clock.
-              const float x = v[j];
-              if (gr == 6) low[h + j] = x * 0x1p-15f;
-              if (gr == 5)
-                ev[h + j] = (int64_t)(uint64_t)__float_as_uint(fmaf(x, 0x1p-6f, low[h + j]) + 12582912.f) - kMagic;
-              if (gr == 4) ev[h + j] += (int64_t)__float2int_rn(x) * (1 << 3);
-              if (gr == 3) ev[h + j] += (int64_t)__float2int_rn(x) * (1 << 12);
-              if (gr == 2) ev[h + j] += (int64_t)__float2int_rn(x) * (1 << 21);
-              if (gr == 1) ev[h + j] += (int64_t)__float2int_rn(x) * (1 << 30);
-              if (gr == 0) ev[h + j] += (int64_t)(((uint64_t)__float_as_uint(x + 12582912.f) - kMagic) << 39);
-            } else {
-              ev[h + j] = v[j];
-            }
-          }
-        }
+        for (int h = 0; h < kW; h += 16) tc::tmem_ld16(tl + (uint32_t)(slot * kCols + h), ev + h);
         tc::fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&accempty[slot]);
@@ -627,15 +707,55 @@ __global__ void __launch_bounds__((Form<T>::EpiWarps + 1 + kLoadWarps) * 32, For
       if (ok && tid == 0 && c + 1 < nchunk) load_list(c + 1);
     }
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
-    for (int i = tid; i < g.nb; i += kEpi) {
+    bool finish = true;
+    if (!whole) {
+      // this piece's sums out; the string's last CTA adds the pieces
+      const int row = piece / g.split;
+      for (int i = tid; i < g.nb; i += kEpi) {
+        g.part_lo[(int64_t)piece * g.nb + i] = lo[i];
+        g.part_hi[(int64_t)piece * g.nb + i] = hi[i];
+      }
+      __threadfence();
+      asm volatile("bar.sync 1, %0;\n" ::"r"(kEpi) : "memory");
+      if (tid == 0) {
+        unsigned* cnt = g.part_count + 2 * row;
+        if (!ok) atomicOr(cnt + 1, 1u);
+        __threadfence();
+        int state = atomicAdd(cnt, 1u) == (unsigned)g.split - 1 ? 1 : 0;
+        __threadfence();
+        if (state) {
+          if (atomicExch(cnt + 1, 0u)) state = 2;
+          *cnt = 0u;
+        }
+        last_ = state;
+      }
+      asm volatile("bar.sync 1, %0;\n" ::"r"(kEpi) : "memory");
+      finish = last_ > 0;
+      if (last_ == 2) ok = false;
+      if (finish) {
+        __threadfence();
+        const int64_t p0 = (int64_t)row * g.split * g.nb;
+        for (int i = tid; i < g.nb; i += kEpi) {
+          uint64_t sl = 0;
+          int32_t sh = 0;
+          for (int k = 0; k < g.split; ++k) {
+            const uint64_t a = __ldcg(g.part_lo + p0 + (int64_t)k * g.nb + i);
+            sl += a;
+            sh += __ldcg(g.part_hi + p0 + (int64_t)k * g.nb + i) + (sl < a ? 1 : 0);
+          }
+          lo[i] = sl;
+          hi[i] = sh;
+        }
+      }
+    }
+    for (int i = tid; finish && i < g.nb; i += kEpi) {
       const int64_t at = Ia * g.nb + i;
       if constexpr (kF64) {
         // the integer once to FP64, then its unit
         const int64_t l = (int64_t)lo[i];
         const int32_t h = hi[i];
-        double v = (double)l;
-        if ((int64_t)h != (l >> 63)) v = (double)h * 0x1p64 + (double)(uint64_t)l;
-        v = scale2(v, min(mexp[0], mexp[1]) - kUnit);
+        const int e = min(mexp[0], mexp[1]) - kUnit;
+        double v = (int64_t)h == (l >> 63) ? whole_scaled(l, e) : scale2((double)h * 0x1p64 + (double)(uint64_t)l, e);
         v += fma(g.D[at], g.C[at], g.sigma[at]);
         g.sigma[at] = ok ? v : nan;
       } else {
@@ -769,13 +889,30 @@ struct DenseArgs {
   double* out;
   const int* bad;
   unsigned* fault;
+  int zsplit;                  // CTAs per tile, each with a range of the K blocks
+  unsigned long long* zsum;    // their sums [tile][product][column][row] (whole numbers; zero before and after)
+  unsigned* zcount;            // per tile: arrived, failed (zero before and after)
 };
 
+// CTAs per tile: as many as the idle SMs allow, with two K blocks each at
+// least.  252 strings are eight tiles of sixteen blocks: one CTA each 38.8 us,
+// eight each 29 us; 462 are 32 tiles: 58 and 37 us.
+inline int dense_split(int64_t tiles, int nblk, int sms) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(sms / tiles, nblk / 2));
+}
+
+// USE: 0 reads A and keeps it in the collector, 1 takes it from there, 2 for
+// the last time
+template <int USE>
 __device__ __forceinline__ void mma_f16_ss(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(dtmem),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
+#define QDKGB_MMA_SS(op)                                                              \
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"                         \
+               " tcgen05.mma.cta_group::1.kind::f16.collector::a::" op " [%0], %1, %2, %3, p;\n}\n" ::"r"(dtmem), \
+               "l"(a), "l"(b), "r"(idesc), "r"(accumulate))
+  if (USE == 0) QDKGB_MMA_SS("fill");
+  if (USE == 1) QDKGB_MMA_SS("use");
+  if (USE == 2) QDKGB_MMA_SS("lastuse");
+#undef QDKGB_MMA_SS
 }
 
 // warp 0 lane 0 fills a two-stage ring with bulk copies (both operands' seven
@@ -785,7 +922,7 @@ __global__ void __launch_bounds__(kDnThreads, 1) k_dense64(DenseArgs g) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t full[kDnStages], empty[kDnStages], accfull, accempty;
   __shared__ uint32_t tslot;
-  __shared__ int fail_;
+  __shared__ int fail_, last_;
   volatile int* fail = &fail_;
   if (*g.bad) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -805,17 +942,19 @@ __global__ void __launch_bounds__(kDnThreads, 1) k_dense64(DenseArgs g) {
   __syncthreads();
   tc::fence_after();
   const uint32_t tmem = tslot;
-  const int nblk = g.nkb1 + g.nkb2;
+  const int nblk_all = g.nkb1 + g.nkb2;
+  const int blk0 = (int)blockIdx.z * nblk_all / g.zsplit, nblk = ((int)blockIdx.z + 1) * nblk_all / g.zsplit;
   // the flush ranges end at multiples of `flush` blocks of each product and at its last
   auto range_end = [&](int b) {
-    return b < g.nkb1 ? ((b + 1) % g.flush == 0 || b + 1 == g.nkb1)
-                      : ((b - g.nkb1 + 1) % g.flush == 0 || b + 1 == nblk);
+    return (b < g.nkb1 ? ((b + 1) % g.flush == 0 || b + 1 == g.nkb1)
+                       : ((b - g.nkb1 + 1) % g.flush == 0 || b + 1 == nblk_all)) ||
+           b + 1 == nblk;
   };
   if (warp == 0) {
     if (lane == 0) {
-      for (int b = 0; b < nblk; ++b) {
-        const int s = b % kDnStages;
-        if (b >= kDnStages && !wait(&empty[s], (uint32_t)((b / kDnStages - 1) & 1), fail)) break;
+      for (int b = blk0; b < nblk; ++b) {
+        const int l = b - blk0, s = l % kDnStages;
+        if (l >= kDnStages && !wait(&empty[s], (uint32_t)((l / kDnStages - 1) & 1), fail)) break;
         const bool p2 = b >= g.nkb1;
         const int kb = p2 ? b - g.nkb1 : b, nkb = p2 ? g.nkb2 : g.nkb1;
         unsigned char* st = smem + s * (kDnA + kDnB);
@@ -830,10 +969,10 @@ __global__ void __launch_bounds__(kDnThreads, 1) k_dense64(DenseArgs g) {
       constexpr uint32_t idesc = idesc_f16(kDnM, kDnN, 0) & ~(1u << 16);  // both operands K-major
       bool ok = true;
       uint32_t first = 1, ranges = 0;
-      int b = 0;
+      int b = blk0;
       for (; b < nblk; ++b) {
-        const int s = b % kDnStages;
-        ok = __all_sync(0xffffffffu, wait(&full[s], (uint32_t)((b / kDnStages) & 1), fail));
+        const int l = b - blk0, s = l % kDnStages;
+        ok = __all_sync(0xffffffffu, wait(&full[s], (uint32_t)((l / kDnStages) & 1), fail));
         if (ok && first && ranges > 0) ok = __all_sync(0xffffffffu, wait(&accempty, (ranges - 1) & 1, fail));
         if (!ok) break;
         tc::fence_after();
@@ -842,15 +981,25 @@ __global__ void __launch_bounds__(kDnThreads, 1) k_dense64(DenseArgs g) {
         const bool last = range_end(b);
         if (elect_one()) {
           const uint32_t acc0 = first ? 0u : 1u;
+          // each part of A against all its parts of B in turn, so that A is read
+          // from shared memory once per part and not once per product
 #pragma unroll
-          for (int gr = 0; gr < kDnS; ++gr)
+          for (int ks = 0; ks < kDnK / 16; ++ks)
 #pragma unroll
-            for (int i = 0; i <= gr; ++i)
+            for (int i = 0; i < kDnS; ++i) {
+              const uint64_t ai = da + (uint64_t)(i * (kDnM * kDnK * 2 / 16) + ks * 16);
 #pragma unroll
-              for (int ks = 0; ks < kDnK / 16; ++ks)
-                mma_f16_ss(tmem + 64 * gr, da + (uint64_t)(i * (kDnM * kDnK * 2 / 16) + ks * 16),
-                           db + (uint64_t)((gr - i) * (kDnN * kDnK * 2 / 16) + ks * 16), idesc,
-                           (i == 0 && ks == 0) ? acc0 : 1u);
+              for (int j = 0; j < kDnS - i; ++j) {
+                const uint32_t acc = (i == 0 && ks == 0) ? acc0 : 1u, dt = tmem + 64 * (i + j);
+                const uint64_t bj = db + (uint64_t)(j * (kDnN * kDnK * 2 / 16) + ks * 16);
+                if (j == 0)
+                  mma_f16_ss<0>(dt, ai, bj, idesc, acc);
+                else if (j < kDnS - 1 - i)
+                  mma_f16_ss<1>(dt, ai, bj, idesc, acc);
+                else
+                  mma_f16_ss<2>(dt, ai, bj, idesc, acc);
+              }
+            }
           tc::commit(&empty[s]);
           if (last) tc::commit(&accfull);
         }
@@ -863,7 +1012,7 @@ __global__ void __launch_bounds__(kDnThreads, 1) k_dense64(DenseArgs g) {
         __syncwarp();
         tc::mbar_wait(&accfull, ranges & 1, kSpin);
         // copies in flight: the stages filled or being filled
-        for (int f = b + 1; f < nblk && f < b + kDnStages; ++f)
+        for (int f = b - blk0 + 1; f < nblk - blk0 && f < b - blk0 + kDnStages; ++f)
           tc::mbar_wait(&full[f % kDnStages], (uint32_t)((f / kDnStages) & 1), kSpin);
       }
     }
@@ -880,7 +1029,11 @@ __global__ void __launch_bounds__(kDnThreads, 1) k_dense64(DenseArgs g) {
       v[j] = 0.;
       acc[j] = 0;
     }
-    for (int b = 0; b < nblk; ++b) {
+    unsigned long long* z1 =
+        g.zsum + ((int64_t)(rb * gridDim.x + nbk) * 2 * kDnN + 32 * half) * kDnM + q * 32 + lane;
+    unsigned long long* z2 = z1 + kDnN * kDnM;
+    const int er1 = row < g.M ? g.ea1[row] - kDnUnit : 0, er2 = row < g.M ? g.ea2[row] - kDnUnit : 0;
+    for (int b = blk0; b < nblk; ++b) {
       if (!range_end(b)) continue;
       if (ok) ok = __all_sync(0xffffffffu, wait(&accfull, ranges & 1, fail));
       ++ranges;
@@ -908,17 +1061,68 @@ __global__ void __launch_bounds__(kDnThreads, 1) k_dense64(DenseArgs g) {
       __syncwarp();
       if (lane == 0) mbar_arrive(&accempty);
       if (b + 1 == g.nkb1 || b + 1 == nblk) {
-        const int* ea = b + 1 == g.nkb1 ? g.ea1 : g.ea2;
-        const int* eb = b + 1 == g.nkb1 ? g.eb1 : g.eb2;
-        const int er = row < g.M ? ea[row] - kDnUnit : 0;
+        const bool second = b >= g.nkb1;
+        const int er = second ? er2 : er1;
+        const int* eb = second ? g.eb2 : g.eb1;
+        unsigned long long* z = second ? z2 : z1;
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
-          if (acc[j] != 0 && c0 + j < g.N) v[j] += scale2((double)acc[j], er + eb[c0 + j]);
+          if (acc[j] != 0 && row < g.M && c0 + j < g.N) {
+            if (g.zsplit > 1)
+              atomicAdd(z + j * kDnM, (unsigned long long)acc[j]);
+            else
+              v[j] += whole_scaled(acc[j], er + eb[c0 + j]);
+          }
           acc[j] = 0;
         }
       }
     }
-    if (row < g.M)
+    bool finish = true;
+    if (g.zsplit > 1) {
+      // the tile's last CTA takes the sums and leaves zeros
+      __threadfence();
+      asm volatile("bar.sync 1, %0;\n" ::"r"(kDnEpi * 32) : "memory");
+      if (tid == 64) {
+        unsigned* cnt = g.zcount + 2 * (rb * gridDim.x + nbk);
+        if (!ok) atomicOr(cnt + 1, 1u);
+        __threadfence();
+        int state = atomicAdd(cnt, 1u) == (unsigned)g.zsplit - 1 ? 1 : 0;
+        __threadfence();
+        if (state) {
+          if (atomicExch(cnt + 1, 0u)) state = 2;
+          *cnt = 0u;
+        }
+        last_ = state;
+      }
+      asm volatile("bar.sync 1, %0;\n" ::"r"(kDnEpi * 32) : "memory");
+      finish = last_ > 0;
+      if (last_ == 2) ok = false;
+      if (finish && row < g.M) {
+        __threadfence();
+#pragma unroll
+        for (int j0 = 0; j0 < 32; j0 += 8) {
+          // eight columns' loads together (columns past N hold zeros)
+          int64_t s1[8], s2[8];
+          int b1[8], b2[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            s1[j] = (int64_t)__ldcg(z1 + (j0 + j) * kDnM);
+            s2[j] = (int64_t)__ldcg(z2 + (j0 + j) * kDnM);
+            const int col = min(c0 + j0 + j, g.N - 1);
+            b1[j] = g.eb1[col];
+            b2[j] = g.eb2[col];
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            if (s1[j] != 0) v[j0 + j] += whole_scaled(s1[j], er1 + b1[j]);
+            if (s2[j] != 0) v[j0 + j] += whole_scaled(s2[j], er2 + b2[j]);
+            z1[(j0 + j) * kDnM] = 0ull;
+            z2[(j0 + j) * kDnM] = 0ull;
+          }
+        }
+      }
+    }
+    if (finish && row < g.M)
 #pragma unroll
       for (int j = 0; j < 32; ++j)
         if (c0 + j < g.N)

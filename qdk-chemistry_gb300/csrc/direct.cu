@@ -153,7 +153,9 @@ struct DirectSigma {
   int ct_mr = 0, ct_R = 0, ct_kpad = 0, ct_nbp = 0, ct_seg = 0;
   int dn_flush = 0;
   unsigned* ct_fault = nullptr;  // g_tc_fault's device address
-  DeviceBuffer ct_rs, ct_walk, ct_segs, ct_V32, ct_V64, ct_C, ct_rexp, ct_cexp, ct_flag;
+  DeviceBuffer ct_rs, ct_walk, ct_segs, ct_V32, ct_V64, ct_C, ct_rexp, ct_cexp, ct_flag, ct_part, ct_count, dn_zsum, dn_zcount;
+  int dn_z = 1;
+  ct::RowPlan rows{0, 1};
   DeviceBuffer dn_Ha, dn_Hb, dn_ea, dn_eb, dn_CA, dn_CB;
   // batched CASCI over instances of this space (direct_batch_*): per-instance
   // FP32 value tables and their dense same-spin matrices; bform -1 until the
@@ -173,7 +175,7 @@ void free_direct(Context* c) {
                           &d->Haa, &d->HbbT, &d->bsAa, &d->bWa, &d->bdva, &d->bsAb, &d->bWb, &d->bdvb, &d->bV2,
                           &d->bHaa, &d->bHbbT, &d->HaaS, &d->HbbS, &d->XA, &d->XB, &d->bHaaS, &d->bHbbS,
                           &d->bXA, &d->bXB, &d->ct_rs, &d->ct_walk, &d->ct_segs, &d->ct_V32, &d->ct_V64, &d->ct_C,
-                          &d->ct_rexp, &d->ct_cexp, &d->ct_flag, &d->dn_Ha, &d->dn_Hb, &d->dn_ea, &d->dn_eb,
+                          &d->ct_rexp, &d->ct_cexp, &d->ct_flag, &d->ct_part, &d->ct_count, &d->dn_zsum, &d->dn_zcount, &d->dn_Ha, &d->dn_Hb, &d->dn_ea, &d->dn_eb,
                           &d->dn_CA, &d->dn_CB})
     dev_free(c, *b);
   delete d;
@@ -1216,7 +1218,7 @@ static void ct_sigma64(Context* c, const double* x, double* y);
 template <typename T>
 static ct::Args<T> ct_args(Context* c, DirectSigma* d, const T* x, T* y);
 template <typename T>
-static void ct_launch(Context* c, const ct::Args<T>& g, int B);
+static void ct_launch(Context* c, const ct::Args<T>& g);
 
 template <typename T>
 static void direct_sigma_t(Context* c, const T* x, T* y) {
@@ -1306,7 +1308,7 @@ static void direct_sigma_t(Context* c, const T* x, T* y) {
           ct::k_ct_split32<<<(unsigned)na, 256, 0, c->stream>>>((int)nb, d->ct_nbp, g.part, (const float*)x,
                                                                 (uint16_t*)d->ct_C.ptr, 0, 0, nullptr);
           QDKGB_CHECK_LAUNCH();
-          ct_launch(c, g, 1);
+          ct_launch(c, g);
           return;
         }
         if (form == 1) {
@@ -1424,7 +1426,7 @@ static void ct_values(Context* c, DirectSigma* d) {
     // a capped context keeps the memory it had for a Davidson workspace of any
     // size: the 16-bit operands only beside that
     const double need = 14.0 * na * d->ct_nbp + (double)(ta * ct::kDnA) * (nkb1 + nkb2) +
-                        (double)(tb * ct::kDnB) * (nkb1 + nkb2) + 64.0 * (na + nb);
+                        (double)(tb * ct::kDnB) * (nkb1 + nkb2) + 64.0 * (na + nb) + 12.0 * c->sm_count * nb + 131072.0 * c->sm_count;
     if (need + 8.0 * na * nb * 530 > (double)(c->dev_limit - c->dev_bytes)) return;
   }
   int* flag = dev_array<int>(c, d->ct_flag, 2);  // [0] asymmetric integrals, [1] non-finite vector
@@ -1444,6 +1446,11 @@ static void ct_values(Context* c, DirectSigma* d) {
                                                  d->ct_R, v64);
   QDKGB_CHECK_LAUNCH();
   dev_array<uint16_t>(c, d->ct_C, (size_t)(7 * na * d->ct_nbp));
+  d->rows = ct::row_plan((int)na, d->ct_nbp / ct::kCols, c->sm_count);
+  const int64_t split_rows = na - d->rows.full, pieces = split_rows * d->rows.split;
+  dev_array<uint64_t>(c, d->ct_part, (size_t)(pieces * nb + (pieces * nb + 1) / 2));
+  unsigned* count = dev_array<unsigned>(c, d->ct_count, (size_t)(2 * split_rows));
+  QDKGB_CUDA(cudaMemsetAsync(count, 0, (size_t)(2 * split_rows) * 4, c->stream));
   void* fault = nullptr;
   QDKGB_CUDA(cudaGetSymbolAddress(&fault, g_tc_fault));
   d->ct_fault = (unsigned*)fault;
@@ -1468,6 +1475,15 @@ static void ct_values(Context* c, DirectSigma* d) {
       (const int32_t*)B.svo.ptr, (const double*)B.sA64.ptr, ct::kDnN, nkb2, Hb, eb);
   QDKGB_CHECK_LAUNCH();
   set_max_dynamic_smem((const void*)ct::k_dense64, ct::kDnStages * (ct::kDnA + ct::kDnB));
+  const int64_t tiles = ta * ((nb + ct::kDnN - 1) / ct::kDnN);
+  d->dn_z = ct::dense_split(tiles, nkb1 + nkb2, c->sm_count);
+  if (d->dn_z > 1) {
+    const int64_t zwords = tiles * 2 * ct::kDnM * ct::kDnN;
+    dev_array<unsigned long long>(c, d->dn_zsum, (size_t)zwords);
+    dev_array<unsigned>(c, d->dn_zcount, (size_t)(2 * tiles));
+    QDKGB_CUDA(cudaMemsetAsync(d->dn_zsum.ptr, 0, (size_t)zwords * 8, c->stream));
+    QDKGB_CUDA(cudaMemsetAsync(d->dn_zcount.ptr, 0, (size_t)(2 * tiles) * 4, c->stream));
+  }
   d->use64 = true;
 }
 
@@ -1502,14 +1518,19 @@ static ct::Args<T> ct_args(Context* c, DirectSigma* d, const T* x, T* y) {
   g.sigma = y;
   g.bad = (const int*)d->ct_flag.ptr + 1;
   g.fault = d->ct_fault;
+  g.full = f64 ? d->rows.full : g.na;
+  g.split = d->rows.split;
+  g.part_lo = (uint64_t*)d->ct_part.ptr;
+  g.part_hi = (int32_t*)(g.part_lo + (int64_t)(g.na - g.full) * g.split * g.nb);
+  g.part_count = (unsigned*)d->ct_count.ptr;
   return g;
 }
 template <typename T>
-static void ct_launch(Context* c, const ct::Args<T>& g, int B) {
+static void ct_launch(Context* c, const ct::Args<T>& g) {
   const ct::Smem<T> s(g.kpad, g.R, g.nb, g.seg_bytes);
   auto go = [&](auto kern) {
     set_max_dynamic_smem((const void*)kern, s.total);
-    kern<<<dim3((unsigned)g.na, (unsigned)B), (ct::Form<T>::EpiWarps + 1 + ct::kLoadWarps) * 32, s.total,
+    kern<<<(unsigned)(g.full + (g.na - g.full) * g.split), (ct::Form<T>::EpiWarps + 1 + ct::kLoadWarps) * 32, s.total,
            c->stream>>>(g);
   };
   switch (g.kpad / 16) {
@@ -1547,11 +1568,12 @@ static void ct_sigma64(Context* c, const double* x, double* y) {
   QDKGB_CHECK_LAUNCH();
   ct::DenseArgs q{na, nb, nkb1, nkb2, d->dn_flush, (const uint16_t*)d->dn_Ha.ptr, (const uint16_t*)d->dn_CB.ptr,
                   (const uint16_t*)d->dn_CA.ptr, (const uint16_t*)d->dn_Hb.ptr, (const int*)d->dn_ea.ptr, cexp, rexp,
-                  (const int*)d->dn_eb.ptr, y, bad, g.fault};
-  ct::k_dense64<<<dim3((unsigned)tb, (unsigned)ta), ct::kDnThreads, ct::kDnStages * (ct::kDnA + ct::kDnB),
+                  (const int*)d->dn_eb.ptr, y, bad, g.fault, d->dn_z, (unsigned long long*)d->dn_zsum.ptr,
+                  (unsigned*)d->dn_zcount.ptr};
+  ct::k_dense64<<<dim3((unsigned)tb, (unsigned)ta, (unsigned)d->dn_z), ct::kDnThreads, ct::kDnStages * (ct::kDnA + ct::kDnB),
                   c->stream>>>(q);
   QDKGB_CHECK_LAUNCH();
-  ct_launch(c, g, 1);
+  ct_launch(c, g);
   ct::PlainArgs p{na,
                   nb,
                   d->n,
@@ -1743,7 +1765,7 @@ static void build_mm_tables(Context* c, DirectSigma* d) {
 // parts.  Measured, whole sigma, before -> after: FP32 12.9 thousand
 // determinants (9, 2, 5) 27 -> 31 us, 63.5 thousand (10, 5, 5) 48 -> 45 us,
 // 854 thousand (12, 6, 6) 366 -> 193 us; FP64 4.9 thousand 65 -> 71 us, 63.5
-// thousand 168 -> 126 us, 854 thousand 3.76 -> 0.72 ms.
+// thousand 168 -> 103 us, 854 thousand 3.76 -> 0.58 ms.
 constexpr int64_t kCtMinDets = 32768;
 
 // Structure of the contraction from 16-bit parts (contract.cuh): the pair
@@ -1882,9 +1904,10 @@ static void build_ct_tables(Context* c, DirectSigma* d) {
   const int nkb = (int)((std::max(A.nstr, nb) + ct::kDnK - 1) / ct::kDnK);
   for (int f = nkb; f >= 1; f = f > 1 ? (f + 1) / 2 : 0) {
     int worst = 0;
-    for (const SpinTables* t : {&A, &B}) {
+    for (int spin = 0; spin < (d->same ? 1 : 2); ++spin) {
+      const SpinTables* t = spin ? &B : &A;
       std::vector<int> h;
-      for (int64_t i = 0; i < t->nstr; ++i) {
+      for (int64_t i = 0; i < t->nstr && worst <= ct::kDnMaxRow; ++i) {
         h.assign((size_t)(t->nstr / (f * ct::kDnK)) + 1, 0);
         for (int m = 0; m < t->nd; ++m) worst = std::max(worst, ++h[t->h_dJ[(size_t)i * t->nd + m] / (f * ct::kDnK)]);
         for (int m = 0; m < t->ns; ++m)
@@ -2006,16 +2029,15 @@ bool attach_direct_fp32(Context* c) {
   return d->mm;
 }
 
-// Stored complete spaces from this size up take their FP64 sigma through the
-// 16-bit digits as well (the matrix stays for the exports): 854 thousand
-// determinants 2.82 ms from the slab, 0.72 ms; 63.5 thousand 138 and 126 us,
-// where the tables' set-up (0.3 ms and more on the host) would not pay.
-constexpr int64_t kCtStoredMinDets = (int64_t)1 << 17;
-
+// Stored complete spaces of kCtMinDets determinants and more take their FP64
+// sigma through the 16-bit digits as well (the matrix stays for the exports):
+// 854 thousand determinants 2.82 ms from the slab, 0.58 ms; 63.5 thousand 138
+// and 103 us, and a new space's first sigma times no plans (a 10e10o gradient,
+// 73 sigmas: 30.9 and 26.7 ms).
 bool attach_direct_fp64(Context* c, double thresh, bool prepared) {
   // the digits hold every element: only where the threshold is no more than
   // the rounding of the largest ones
-  if (c->dets.ndets < kCtStoredMinDets || thresh > std::numeric_limits<double>::epsilon()) return false;
+  if (c->dets.ndets < kCtMinDets || thresh > std::numeric_limits<double>::epsilon()) return false;
   size_t fr = 0, tot = 0;
   QDKGB_CUDA(cudaMemGetInfo(&fr, &tot));
   // beside a Davidson workspace of any size
