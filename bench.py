@@ -351,7 +351,12 @@ def run_ours(args):
     else:
         bytes32 = nnz * 8 + (N + 1) * 8 + N * 4 + N * 4
         kern32 = "k_spmv_csr<float> (FP32 sigma, CSR)"
-    if lay64 == capi.OP_SLAB:
+    if lay64 == capi.OP_SLAB and not ctx.sigma_plan(capi.PREC_FP64)[1]:
+        # no slab plan was timed: the direct contraction's digits serve
+        bytes64 = None
+        kern64 = ("k_contract<double> + k_dense64 (FP64 sigma from 16-bit digits on tcgen05; the stored slab serves "
+                  "the exports)")
+    elif lay64 == capi.OP_SLAB:
         bytes64 = stored64 * 8 + N * 8 + N * 8
         kern64 = "k_slab_sigma<1> (FP64 sigma, slab layout; FP64-pipe bound)"
     else:
@@ -360,29 +365,30 @@ def run_ours(args):
     roof = None
     if lay32 in (capi.OP_SLAB_DIRECT32, capi.OP_DIRECT):
         # FLOPs of one FP32 direct sigma as formulated: the contraction forms
-        # E (rows: the n(n-1) pairs, n W rows, one string row; K: the alpha
+        # E (rows: the n(n-1)/2 pairs, n W rows, one string row; K: the alpha
         # singles and the own row) for every beta string; the same-spin part
         # as two dense products (or the element-wise kernels, fewer FLOPs)
         ka = NEL // 2
         na_s = math.comb(NORB, ka)
         nsa = ka * (NORB - ka)
-        rows = NORB * (NORB - 1) + NORB + 1
+        rows = NORB * (NORB - 1) // 2 + NORB + 1
         flops = 2.0 * na_s * rows * (nsa + 1) * na_s
         plan = ctx.direct_plan()
         if plan.get("dense"):
             flops += 2.0 * 2 * na_s ** 3
         if plan.get("contraction") == "tensor":
-            # TF32 x 3 on tcgen05: the tensor pipe runs three TF32 products per
-            # FP32 product; its dense TF32 rate is half the measured bf16 rate
-            tf32_peak = _bf16_peak() / 2
-            achieved = 3 * flops / t_spmv32 / 1e12
-            kern32 = ("FP32 direct sigma on the tensor cores: k_ds_opposite_tc (opposite-spin doubles and every "
-                      "single excitation as one tcgen05 TF32x3 contraction per alpha string) + k_tc_gemm2b (the "
-                      "same-spin string-only part as two dense tcgen05 TF32x3 products)")
-            roof = {"bound": "tensor", "kernel": kern32, "achieved": achieved, "peak": tf32_peak,
-                    "unit": "TFLOP/s", "frac": achieved / tf32_peak,
-                    "peak_source": "measured bf16 dense rate / 2 (TF32), of measured", "traffic": None,
-                    "algorithmic_flops": flops, "tensor_flops": 3 * flops, "launch_ms": t_spmv32 * 1e3,
+            # six products of bfloat16 parts per FP32 product in the
+            # contraction, three of TF32 (half the bf16 rate) in the dense
+            # products: six bf16 products' time either way
+            bf16_peak = _bf16_peak()
+            achieved = 6 * flops / t_spmv32 / 1e12
+            kern32 = ("FP32 direct sigma on the tensor cores: k_contract<float> (opposite-spin doubles and every "
+                      "single excitation as one tcgen05 contraction per alpha string, from bfloat16 parts) + "
+                      "k_tc_gemm2b (the same-spin string-only part as two dense tcgen05 TF32x3 products)")
+            roof = {"bound": "tensor", "kernel": kern32, "achieved": achieved, "peak": bf16_peak,
+                    "unit": "TFLOP/s", "frac": achieved / bf16_peak,
+                    "peak_source": "measured bf16 dense rate, of measured", "traffic": None,
+                    "algorithmic_flops": flops, "tensor_flops": 6 * flops, "launch_ms": t_spmv32 * 1e3,
                     "plan": plan}
         else:
             fp32_peak = 152 * 128 * 2 * 2.07e9 / 1e12
@@ -394,7 +400,7 @@ def run_ours(args):
         achieved32 = None
     else:
         achieved32 = bytes32 / t_spmv32 / 1e9
-    achieved64 = bytes64 / t_spmv64 / 1e9
+    achieved64 = bytes64 / t_spmv64 / 1e9 if bytes64 else None
     traffic = None
     tp = os.path.join(ROOT, "profiles", "spmv_traffic.json")
     if os.path.exists(tp) and lay32 == capi.OP_SLAB:
@@ -443,7 +449,8 @@ def run_ours(args):
                              "peak": peak, "unit": "GB/s", "frac": achieved32 / peak, "peak_source": peak_kind,
                              "traffic": traffic, "algorithmic_bytes": bytes32, "launch_ms": t_spmv32 * 1e3},
         "operator_mixed": capi.LAYOUT_NAMES.get(lay32),
-        "spmv_fp64": {"kernel": kern64, "achieved_gbs": achieved64, "frac": achieved64 / peak,
+        "spmv_fp64": {"kernel": kern64, "achieved_gbs": achieved64,
+                      "frac": achieved64 / peak if achieved64 else None,
                       "launch_ms": t_spmv64 * 1e3, "algorithmic_bytes": bytes64},
         "sigma_autotune": {"fp32": dict(zip(("segments", "candidates_ms", "kernel", "kernel_candidates_ms"),
                                             ctx.sigma_plan(capi.PREC_MIXED, with_kernel=True))),

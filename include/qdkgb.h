@@ -93,8 +93,8 @@ int qdkgb_operator_layout(const qdkgb_context* ctx, int* layout, int64_t* stored
  * QDKGB_LAYOUT_SLAB_DIRECT32; no counterpart in the reference):
  * *contraction 0 the element-wise walk, 1 the opposite-spin doubles and the
  * single excitations as one FP32 contraction per alpha string on the FMA
- * pipe, 2 the same with the contraction on the tensor cores (tcgen05, TF32
- * x 3); *dense the same-spin part's form, -1 until the first FP32 sigma
+ * pipe, 2 the same with the contraction on the tensor cores (tcgen05: six
+ * products of bfloat16 parts, or TF32 x 3 where those do not apply); *dense the same-spin part's form, -1 until the first FP32 sigma
  * times the forms, 0 element-wise kernels, 1 two dense products (tensor
  * cores unless QDKGB_DIRECT_TC=0); form_ms[4] the times (ms) of the
  * same-spin forms (element-wise, dense) and of the contractions (FMA pipe,
@@ -183,7 +183,9 @@ int qdkgb_build_operator(qdkgb_context* ctx, double thresh, int storage, int max
  * candidate count, one untimed and three timed sigmas each, and keeps the
  * fastest.  *segments receives the count in use (0: no complete-space
  * sigma); with ncand (in: capacity, out: candidates tried) the candidates'
- * counts and mean milliseconds, empty before the first sigma.  For the FP32
+ * counts and mean milliseconds, empty before the first sigma and where the
+ * precision's sigma does not run from the slab (FP64 from 32,768 determinants
+ * up: the direct contraction's 16-bit digits).  For the FP32
  * sigma the tuner also times the TMA-fed kernel (slab rows streamed into
  * shared memory by bulk copies) and the register-fed kernel with eight and
  * with sixteen positions in flight per thread on every candidate: *kernel

@@ -168,8 +168,8 @@ static int64_t cas_row_elements(int n, int ka, int kb) {
 // mixed-precision solves (QDKGB_H_SPLIT32): their FP32 sigma is the direct
 // contraction whatever is stored, so a stored FP64 matrix would serve only the
 // few full-precision refreshes of the solve, and emitting it costs more than
-// recomputing them (853,776 determinants: 9.3 ms of emission, refreshes of
-// 2.8 ms from the stored matrix against 3.75 ms recomputed, four refreshes).
+// recomputing them (853,776 determinants: 9.3 ms of emission against four
+// refreshes of 0.58 ms).
 constexpr int64_t kMixedDirectMinDets = (int64_t)1 << 17;
 
 // The stored Hamiltonian when it fits in the device memory available to this
