@@ -926,6 +926,15 @@ struct Dav {
   EigWarm* warm = nullptr;  // the projected problem's state from size to size
   cudaStream_t st;
 
+  // blocks of the FP64 row sums over the basis: a tile each, so that the
+  // hardware evens them out over the SMs (853,776 rows, Ritz step 221 -> 194
+  // us, update 102 -> 96; the double-float kernels lose by it, 73 -> 81, and
+  // keep the resident wave, as does a steady solve, whose blocks add the norms
+  // in its order)
+  int row_blocks() const {
+    return steady ? nb : (int)std::max<int64_t>(1, std::min<int64_t>((n + kVecTile - 1) / kVecTile, (int64_t)sm_count * 16));
+  }
+
   unsigned* counts() { return (unsigned*)(small + kSlotCount); }
 
   double* col(double* base, int64_t j) { return base + (size_t)j * n; }
@@ -993,11 +1002,11 @@ struct Dav {
     if (!steady) {
       double* nrm = small + kSlotNrm;
       multidot(V, K, w, small, 1, small + kSlotW2);
-      k_gemv_rows<true, true><<<nb, kVecThreads, 0, st>>>(V, n, K, small, 1, w, n, nullptr, small + kSlotW2,
+      k_gemv_rows<true, true><<<row_blocks(), kVecThreads, 0, st>>>(V, n, K, small, 1, w, n, nullptr, small + kSlotW2,
                                                           small + kSlotSkip, partial, counts(), nrm);
       QDKGB_CHECK_LAUNCH();
       multidot(V, K, w, small, 1, nullptr, small + kSlotSkip);
-      k_gemv_rows<true, true><<<nb, kVecThreads, 0, st>>>(V, n, K, small, 1, w, n, small + kSlotSkip, nullptr, nullptr,
+      k_gemv_rows<true, true><<<row_blocks(), kVecThreads, 0, st>>>(V, n, K, small, 1, w, n, small + kSlotSkip, nullptr, nullptr,
                                                           partial, counts(), nrm);
       QDKGB_CHECK_LAUNCH();
       return;
@@ -1066,7 +1075,7 @@ struct Dav {
   // stored preconditioned with the diagonal D (the next direction before
   // orthogonalisation)
   void ritz_residual(int k, double* R, double min_abs) {
-    k_ritz_residual<<<nb, kVecThreads, 0, st>>>(V, AV, n, k, evec, eval, X, R, n, D, min_abs, partial, counts(),
+    k_ritz_residual<<<row_blocks(), kVecThreads, 0, st>>>(V, AV, n, k, evec, eval, X, R, n, D, min_abs, partial, counts(),
                                                 small + kSlotRes, small + kSlotFlag);
     QDKGB_CHECK_LAUNCH();
   }
