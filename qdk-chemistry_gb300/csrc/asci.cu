@@ -196,8 +196,9 @@ __device__ __forceinline__ void hll_add(unsigned* reg, uint64_t qa, uint64_t qb)
 
 // What a CTA holds of its core determinant, sized by the determinant's own
 // counts: singles as (occupied, virtual, sign) and their two G2 elements,
-// pairs of occupied and of virtual orbitals.  At most 46 KB (64 orbitals,
-// half of them occupied).
+// pairs of occupied and of virtual orbitals, and before them the terms of the
+// diagonal element.  41 KB for 64 orbitals half occupied, 105 KB at most (all
+// of them occupied).
 __host__ __device__ inline size_t asci_smem(bool count, int n, int ka, int kb, bool just_singles) {
   const size_t ns = (size_t)ka * (n - ka) + (size_t)kb * (n - kb);
   const size_t np = just_singles ? 0
@@ -518,6 +519,10 @@ EnumShape enum_shape(const Context* c, CoreArgs& A, const uint64_t* ca, const ui
   A.nslice = (int)std::max<int64_t>(1, std::min<int64_t>(fill, (rows + kAsciWarps - 1) / kAsciWarps));
   if (A.ncore * A.nslice > 0x7fffffff) throw Error(QDKGB_ERR_UNSUPPORTED, "ASCI: more than 2^31 core determinants");
   e.grid = (unsigned)(A.ncore * A.nslice);
+  // above the default 48 KB only from about 40 electrons of each spin (their
+  // diagonal's terms)
+  set_max_dynamic_smem((const void*)k_asci_enum<true>, (int)e.smem_count);
+  set_max_dynamic_smem((const void*)k_asci_enum<false>, (int)e.smem);
   return e;
 }
 

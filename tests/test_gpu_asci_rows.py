@@ -34,7 +34,8 @@ def _wfn(pkg, norb, na, nb, nd, seed):
 
 
 @pytest.mark.parametrize("norb,na,nb,nd", [(5, 1, 0, 3), (6, 0, 2, 4), (4, 4, 1, 2), (7, 3, 2, 25), (9, 5, 4, 40),
-                                           (12, 2, 6, 7), (33, 2, 1, 5), (40, 3, 3, 2), (64, 1, 1, 3)])
+                                           (12, 2, 6, 7), (33, 2, 1, 5), (40, 3, 3, 2), (64, 1, 1, 3), (48, 40, 40, 2),
+                                           (64, 62, 63, 2)])
 def test_search_and_pt2_match_oracle(capi, pkg, oracle, norb, na, nb, nd):
     T, V, _ = pkg.integrals.synthetic_integrals(norb, 2 * norb, 77 + norb)
     H = oracle.Hamiltonian(T, V)
